@@ -124,6 +124,15 @@ __device__ __forceinline__ int64_t sample_position(int64_t idx, int64_t n) {
   return start + (int64_t)(((uint64_t)hashed * (uint64_t)(end - start)) >> 32);
 }
 
+// A word that a kernel still running when this one was scheduled may have written, read behind
+// cudaGridDependencySynchronize().  Such data must not be reached through `const __restrict__`
+// parameters: those loads count as invariant, and the compiler may move them ahead of the wait.
+__device__ __forceinline__ uint32_t load_dependent_u32(const void* p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // Lane mapping in force (host side, process-wide like the reference's import-time
 // config.lane_mapping): 254 or 0.  Set through lct_set_lane_mapping (capi.cu).
 int lane_mask_now();

@@ -1,32 +1,26 @@
 // Field split + fixed-budget Huffman encoder, and the overflow tail compaction.
 //
-// One CTA (256 threads) per codec block; between the prologue and the epilogue
-// every warp runs on its own (see common.cuh: a warp's 32 lanes own one
-// 64-byte segment of every row).  Per half tile of 16 rows, per warp:
-//   row side  - thread = 8 columns of a row pair: 128-bit loads of the BF16
-//               source (requested one half tile ahead), four values at a time
-//               split into exponent bytes -> the warp's shared tile and side
-//               bytes -> lane order, stored 64 bits at a time;
-//   lane side - thread = lane: two byte loads of its exponent pair from the
-//               tile, both (code, length) rows of the shared encode table,
-//               code appended at the lane's bit position; a finished 32-bit
-//               word goes into a shared image of the block's payload by
-//               predicated instructions (encode_core.cuh).
-// At the end the payload image (zero where nothing was written, so the output
-// is deterministic) is copied out with coalesced 128-bit stores, and the
-// block's overflow summary is reduced.
+// One CTA of 128 threads per codec block, thread = two neighbouring lanes (lanes.cuh).  Per row
+// pair a thread has two 32-bit source words (requested a chunk of 8 rows ahead; a warp reads a
+// full 128-byte line per row), splits off the side bytes and stores them (64 bytes per warp and
+// row), looks the four exponents up in the shared encode table and appends two codes to each of
+// its two bit streams (lane_writer.cuh).  Finished words are collected in a shared image of the
+// block's payload (zero where nothing was written, so the output is deterministic), which is
+// copied out at the end with 128-bit stores.
+//
+// A chunk in which some lane of the warp could run out of its bit budget (or already has) takes
+// the checked form of the append; all others carry no per-pair conditions.
 #include <type_traits>
 
 #include "batch.cuh"
 #include "common.cuh"
-#include "encode_core.cuh"
+#include "lane_writer.cuh"
 #include "lct_b200.h"
 
 namespace lct {
 
-// Resident CTAs per SM the encoder is compiled for (register cap = 65536 / 256 / this; five or
-// six were measured slower, 63.5 and 65.7 us against 61.5 for 64 Mi elements).
-constexpr int kEncodeMinCtas = 4;
+// Resident CTAs per SM the encoder is compiled for: as many as the payload image allows.
+constexpr int kEncodeMinCtas = 5;
 
 struct EncodeShape {
   int64_t size;
@@ -39,282 +33,229 @@ struct EncodeShape {
   int lane_mask;  // 254: lane ^ (row & 254) ("swizzle"); 0: "linear"
 };
 
-// Fixed part of the dynamic shared memory; the payload image follows it.
+// How far ahead of the rows in work the source is brought to L2, and in what portions.
+constexpr int kPrefetchRows = 32, kPrefetchPortion = 2 * kChunkRows;
+
+// Shared memory: encode table | scratch | payload image.
 struct __align__(16) EncodeSharedHead {
-  uint2 table[256];                        // x = code bits (LSB first), y = code length
-  uint16_t tile[kWarps][kTilePairs * 32];
-  int scan[36];
+  uint32_t table[256];
+  int scan[16];
 };
 
-// Source values of one row-phase unit: 8 columns of two consecutive rows.
-struct UnitSource {
-  uint4 top, bottom;  // BF16 bits; for precomputed exponent bytes only .x/.y are used
-};
-
-__device__ __forceinline__ uint32_t load_pair_guarded(const uint16_t* src, int64_t at, int64_t numel) {
-  const uint32_t a = at < numel ? src[at] : 0u;
-  const uint32_t b = at + 1 < numel ? src[at + 1] : 0u;
-  return a | (b << 16);
+// Exponent bytes of two columns, spread to where BF16 values hold them.
+__device__ __forceinline__ uint32_t spread_exponents(uint32_t low, uint32_t high) {
+  return (low << 7) | (high << 23);
 }
-
-template <bool kPrecomputed>
-__device__ __forceinline__ UnitSource load_unit(const void* src, int64_t at, int64_t numel,
-                                                bool vector_ok, bool full_block) {
-  UnitSource u;
-  u.top = make_uint4(0, 0, 0, 0);
-  u.bottom = make_uint4(0, 0, 0, 0);
-  if (kPrecomputed) {
-    const uint8_t* bytes = static_cast<const uint8_t*>(src);
-    if (vector_ok && (full_block || at + kLanes + 8 <= numel)) {
-      const uint2 t = __ldcs(reinterpret_cast<const uint2*>(bytes + at));
-      const uint2 b = __ldcs(reinterpret_cast<const uint2*>(bytes + at + kLanes));
-      u.top.x = t.x; u.top.y = t.y; u.bottom.x = b.x; u.bottom.y = b.y;
-    } else {
-      uint32_t* top = &u.top.x;
-      uint32_t* bottom = &u.bottom.x;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        if (at + i < numel) top[i >> 2] |= (uint32_t)bytes[at + i] << (8 * (i & 3));
-        if (at + kLanes + i < numel) bottom[i >> 2] |= (uint32_t)bytes[at + kLanes + i] << (8 * (i & 3));
-      }
-    }
-  } else {
-    const uint16_t* bits = static_cast<const uint16_t*>(src);
-    if (vector_ok && (full_block || at + kLanes + 8 <= numel)) {
-      u.top = __ldcs(reinterpret_cast<const uint4*>(bits + at));
-      u.bottom = __ldcs(reinterpret_cast<const uint4*>(bits + at + kLanes));
-    } else {
-      uint32_t* top = &u.top.x;
-      uint32_t* bottom = &u.bottom.x;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        top[k] = load_pair_guarded(bits, at + 2 * k, numel);
-        bottom[k] = load_pair_guarded(bits, at + kLanes + 2 * k, numel);
-      }
-    }
-  }
-  return u;
-}
-
-// Row side of one half tile (16 rows) for one thread: 8 columns of one row pair - field split,
-// side bytes to global memory in lane order, exponent bytes into the warp's tile.  Cut into
-// slices (the form a lane phase can issue between its lookups); the last slice requests the
-// source of the half tile after this one.
-template <bool kPrecomputed>
-struct EncodeRowSlices {
-  const void* src;
-  uint8_t* side;
-  uint16_t* tile;
-  int64_t logical_numel, row0, block_base;
-  int halves, warp, lane32, lane_mask;
-  bool vector_ok, full_block;
-  int h = 0;           // the half tile whose source is in `source`
-  UnitSource source;
-  uint32_t l03, h03, l47, h47, bl03, bh03, bl47, bh47;
-  uint32_t e_top03, e_top47, e_bot03, e_bot47;
-
-  __device__ __forceinline__ int pair() const { return kHalfPairs * (h & 1) + (lane32 >> 2); }
-  // Request the source rows of half tile `which` (nothing when it does not exist).
-  __device__ __forceinline__ void request(int which) {
-    h = which;
-    if (which >= halves) return;
-    const int64_t row = row0 + kTileRows * (which >> 1) + 2 * pair();
-    const int64_t logical =
-        row * kLanes + 32 * (warp ^ ((int)(row & lane_mask) >> 5)) + 8 * (lane32 & 3);
-    source = load_unit<kPrecomputed>(src, logical, logical_numel, vector_ok, full_block);
-  }
-  template <int k>
-  __device__ __forceinline__ void slice() {
-    const int p = pair();
-    const int in_tile = (2 * p) & lane_mask;
-    const int swapped = (8 * (lane32 & 3)) ^ (in_tile & 0x18);
-    if (kPrecomputed) {
-      if (k == 0) {
-        e_top03 = source.top.x; e_top47 = source.top.y;
-        e_bot03 = source.bottom.x; e_bot47 = source.bottom.y;
-      }
-    } else {
-      const uint32_t q = (uint32_t)(in_tile >> 1) & 3u;
-      uint8_t* s = side + block_base + (int64_t)(kTileRows * (h >> 1) + 2 * p) * kLanes + 32 * warp + swapped;
-      if (k == 0) {
-        const uint4 t = source.top;
-        l03 = prmt(t.x, t.y, 0x6420); h03 = prmt(t.x, t.y, 0x7531);
-        l47 = prmt(t.z, t.w, 0x6420); h47 = prmt(t.z, t.w, 0x7531);
-      }
-      if (k == 1) {
-        const uint4 b = source.bottom;
-        bl03 = prmt(b.x, b.y, 0x6420); bh03 = prmt(b.x, b.y, 0x7531);
-        bl47 = prmt(b.z, b.w, 0x6420); bh47 = prmt(b.z, b.w, 0x7531);
-      }
-      if (k == 2) {
-        e_top03 = exponent_bytes(l03, h03); e_top47 = exponent_bytes(l47, h47);
-        // Side bytes: column order -> lane order, one 8-byte store per row.
-        const uint32_t s03 = side_bytes(l03, h03), s47 = side_bytes(l47, h47);
-        __stcs(reinterpret_cast<uint2*>(s),
-               make_uint2(prmt(s03, s47, pair_selector_low(q)), prmt(s03, s47, pair_selector_high(q))));
-      }
-      if (k == 3) {
-        e_bot03 = exponent_bytes(bl03, bh03); e_bot47 = exponent_bytes(bl47, bh47);
-        const uint32_t s03 = side_bytes(bl03, bh03), s47 = side_bytes(bl47, bh47);
-        __stcs(reinterpret_cast<uint2*>(s + kLanes),
-               make_uint2(prmt(s03, s47, pair_selector_low(q)), prmt(s03, s47, pair_selector_high(q))));
-      }
-    }
-    if (k == 4) {
-      // tile word for columns (2k, 2k+1): [e_top(2k), e_bot(2k), e_top(2k+1), e_bot(2k+1)];
-      // the unit's group of 8 sits where its lanes are (see tile_slot_xor).
-      *reinterpret_cast<uint4*>(&tile[p * 32 + swapped]) =
-          make_uint4(prmt(e_top03, e_bot03, 0x5140), prmt(e_top03, e_bot03, 0x7362),
-                     prmt(e_top47, e_bot47, 0x5140), prmt(e_top47, e_bot47, 0x7362));
-    }
-    if (k == 5) request(h + 1);
-  }
-  __device__ __forceinline__ void rest() {
-    slice<0>(); slice<1>(); slice<2>(); slice<3>(); slice<4>(); slice<5>();
-  }
-};
 
 // One codec block.  extra_starts and summaries are the tensor's own arrays
 // (summaries holds g.n_blocks entries per row).
 // kLaneMask: the lane mapping as a compile-time constant (254, the default mapping), or -1 to
 // take it from the shape at run time.
 template <bool kPrecomputed, int kLaneMask>
-__device__ __forceinline__ void encode_block(const void* __restrict__ src, bool src_vector_ok,
+struct BlockEncoder {
+  const char* rows;  // the block's first source row
+  uint8_t* side_rows;
+  const EncodeShape& g;
+  int64_t block;
+  uint32_t table;
+  int wide_rows;  // rows, in whole chunks, that may be read as two-value words
+  LaneWriter a, b;
+
+  // What the two lanes append for one row pair, and its side bytes.
+  struct Pair {
+    uint32_t sides, a0, a1, b0, b1;
+  };
+
+  __device__ __forceinline__ Pair look_up(uint32_t top, uint32_t bottom) const {
+    Pair p;
+    uint32_t exponents;
+    split_words(top, bottom, &p.sides, &exponents);
+    p.a0 = encode_entry_of<0>(table, exponents);
+    p.b0 = encode_entry_of<1>(table, exponents);
+    p.a1 = encode_entry_of<2>(table, exponents);
+    p.b1 = encode_entry_of<3>(table, exponents);
+    return p;
+  }
+  __device__ __forceinline__ void store_sides(const Pair& p, int k) const {
+    if (kPrecomputed) return;
+    uint8_t* s = side_rows + (2 * k) * kLanes;
+    __stcs(reinterpret_cast<uint16_t*>(s), (uint16_t)p.sides);
+    __stcs(reinterpret_cast<uint16_t*>(s + kLanes), (uint16_t)(p.sides >> 16));
+  }
+  template <bool kChecked>
+  __device__ __forceinline__ void append(const Pair& p, int step, uint32_t budget_bits) {
+    if (kChecked) {
+      a.append_checked(p.a0, p.a1, step, budget_bits);
+      b.append_checked(p.b0, p.b1, step, budget_bits);
+    } else {
+      a.append(p.a0, p.a1);
+      b.append(p.b0, p.b1);
+    }
+  }
+  // The words of the chunk at step0, all requested together: loads requested one by one between
+  // other work would make every use wait for the latest of them.
+  __device__ __forceinline__ void request(uint32_t (&words)[kChunkRows], int step0) const {
+    if (step0 >= wide_rows) return;
+    const uint32_t offset = chunk_offset<kLaneMask>(block * g.steps, step0, g.lane_mask);
+#pragma unroll
+    for (int row = 0; row < kChunkRows; ++row) {
+      const uint32_t at = chunk_word<kLaneMask>(offset, row >> 1, g.lane_mask);
+      if (kPrecomputed) {
+        const uint32_t bytes = load_ahead_u16(rows + (at >> 1) + row * kLanes);
+        words[row] = spread_exponents(bytes & 255u, bytes >> 8);
+      } else {
+        words[row] = load_ahead_u32(rows + at + row * kRowBytes);
+      }
+    }
+  }
+  // A word by guarded loads: a source of any alignment, a chunk that reaches past the end.
+  __device__ __forceinline__ uint32_t guarded_word(int step0, int k, bool second) const {
+    const int64_t left = g.logical_numel - block * (int64_t)g.block_symbols;
+    const uint32_t offset = chunk_offset<kLaneMask>(block * g.steps, step0, g.lane_mask);
+    const int64_t at = (chunk_word<kLaneMask>(offset, k, g.lane_mask) >> 1) + (2 * k + second) * kLanes;
+    uint32_t low = 0u, high = 0u;
+    if (kPrecomputed) {
+      const uint8_t* p = reinterpret_cast<const uint8_t*>(rows) + at;
+      if (at < left) low = p[0];
+      if (at + 1 < left) high = p[1];
+      return spread_exponents(low, high);
+    }
+    const uint16_t* p = reinterpret_cast<const uint16_t*>(rows) + at;
+    if (at < left) low = p[0];
+    if (at + 1 < left) high = p[1];
+    return low | (high << 16);
+  }
+
+  // The software pipeline: `now` is the row pair to append; while it is appended, the next one's
+  // entries are looked up.  Once a chunk's words (`words`) are looked up, their registers take the
+  // words of the chunk after the next one (`ahead` holds the next one's).
+  template <bool kChecked>
+  __device__ __forceinline__ void step_chunk(int step0, Pair& now, uint32_t (&words)[kChunkRows],
+                                             const uint32_t (&ahead)[kChunkRows], uint32_t budget_bits) {
+#pragma unroll
+    for (int k = 0; k < kChunkPairs; ++k) {
+      const Pair next = k + 1 < kChunkPairs ? look_up(words[2 * k + 2], words[2 * k + 3])
+                                            : look_up(ahead[0], ahead[1]);
+      if (k + 2 == kChunkPairs) request(words, step0 + 2 * kChunkRows);
+      store_sides(now, k);
+      append<kChecked>(now, step0 + 2 * k, budget_bits);
+      now = next;
+    }
+    side_rows += kChunkRows * kLanes;
+  }
+
+  // All rows up to `rows_used`: whole chunks as above, the rest by guarded loads.
+  __device__ __forceinline__ void run(int rows_used, bool prefetches) {
+    const uint32_t budget_bits = (uint32_t)g.fixed_words * 32u;
+    if (wide_rows > 0) {
+      uint32_t even[kChunkRows], odd[kChunkRows];
+      request(even, 0);
+      request(odd, kChunkRows);
+      Pair now = look_up(even[0], even[1]);
+      auto near = [&] { return __any_sync(0xFFFFFFFFu, max(a.bits(), b.bits()) + kChunkBits > budget_bits); };
+#pragma unroll 1
+      for (int step0 = 0; step0 < wide_rows; step0 += 2 * kChunkRows) {
+        if (prefetches && step0 + kPrefetchRows + kPrefetchPortion <= wide_rows)
+          prefetch_l2(rows + (step0 + kPrefetchRows) * kRowBytes, kPrefetchPortion * kRowBytes);
+        if (near())
+          step_chunk<true>(step0, now, even, odd, budget_bits);
+        else
+          step_chunk<false>(step0, now, even, odd, budget_bits);
+        if (step0 + kChunkRows >= wide_rows) break;
+        if (near())
+          step_chunk<true>(step0 + kChunkRows, now, odd, even, budget_bits);
+        else
+          step_chunk<false>(step0 + kChunkRows, now, odd, even, budget_bits);
+      }
+    }
+    const int lane = 2 * threadIdx.x;
+    const int valid_a = valid_steps_of(block, lane, g.steps, g.block_symbols, g.logical_numel, g.lane_mask);
+    const int valid_b = valid_steps_of(block, lane + 1, g.steps, g.block_symbols, g.logical_numel, g.lane_mask);
+#pragma unroll 1
+    for (int step0 = wide_rows; step0 < rows_used; step0 += kChunkRows) {
+      Pair pairs[kChunkPairs];
+#pragma unroll
+      for (int k = 0; k < kChunkPairs; ++k) {
+        Pair& p = pairs[k];
+        p = look_up(guarded_word(step0, k, false), guarded_word(step0, k, true));
+        const int step = step0 + 2 * k;  // padding carries no bits
+        if (step >= valid_a) p.a0 = 0u;
+        if (step + 1 >= valid_a) p.a1 = 0u;
+        if (step >= valid_b) p.b0 = 0u;
+        if (step + 1 >= valid_b) p.b1 = 0u;
+      }
+#pragma unroll
+      for (int k = 0; k < kChunkPairs; ++k) {
+        store_sides(pairs[k], k);
+        append<true>(pairs[k], step0 + 2 * k, budget_bits);
+      }
+      side_rows += kChunkRows * kLanes;
+    }
+  }
+};
+
+template <bool kPrecomputed, int kLaneMask>
+__device__ __forceinline__ void encode_block(const void* __restrict__ src, bool src_word_ok,
                                              uint8_t* __restrict__ side,
                                              uint32_t* __restrict__ encoded,
-                                             const int32_t* __restrict__ shifted_encode,
+                                             const int32_t* shifted_encode,
                                              uint8_t* __restrict__ extra_starts,
                                              int32_t* __restrict__ summaries, const EncodeShape& g_in,
                                              int64_t block) {
   EncodeShape g = g_in;
   if (kLaneMask >= 0) g.lane_mask = kLaneMask;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(128) unsigned char smem_raw[];
   EncodeSharedHead& sh = *reinterpret_cast<EncodeSharedHead*>(smem_raw);
-  uint32_t* payload = reinterpret_cast<uint32_t*>(smem_raw + sizeof(EncodeSharedHead));
+  uint32_t* image = reinterpret_cast<uint32_t*>(smem_raw + sizeof(EncodeSharedHead));
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane32 = tid & 31;
-  const int64_t row0 = block * g.steps;
+  const int tid = threadIdx.x;
   const int64_t block_base = block * (int64_t)g.block_symbols;
-  const bool full_block = block_base + g.block_symbols <= g.logical_numel;
-
-  const int valid = valid_steps_of(block, tid, g.steps, g.block_symbols, g.logical_numel, g.lane_mask);
-  const int budget_bits = g.fixed_words * 32;
-  uint16_t* tile = sh.tile[warp];
-  const uint32_t tile_lane = shared_address(&tile[lane32]);
-  const uint32_t table_address = shared_address(sh.table);
-  uint32_t* payload_column = payload + tid;
-  const SharedWordSink sink{shared_address(payload_column)};
-  uint32_t lo = 0;
-  int pos = 0;
-  int extra_start = -1;  // first overflowing step, -1 = none
-  bool open = true;
-
-  // Rows of this block that hold elements.  Half tiles of pure padding (the tail of a ragged or
-  // tiny tensor) carry no bits; their side bytes are cleared in one sweep after the loop.
-  const int rows_used =
-      full_block ? g.steps : (int)((g.logical_numel - block_base + kLanes - 1) / kLanes);
-  const int halves = (rows_used + kTileRows / 2 - 1) / (kTileRows / 2);
-
-  EncodeRowSlices<kPrecomputed> rows;
-  rows.src = src;
-  rows.side = side;
-  rows.tile = tile;
-  rows.logical_numel = g.logical_numel;
-  rows.vector_ok = src_vector_ok;
-  rows.full_block = full_block;
-  rows.halves = halves;
-  rows.warp = warp;
-  rows.lane32 = lane32;
-  rows.row0 = row0;
-  rows.block_base = block_base;
-  rows.lane_mask = g.lane_mask;
-  rows.request(0);
-  // Everything above is independent of the tensor's center.  The shifted table may come from
-  // a kernel that is still running when this grid was launched with programmatic stream
-  // serialisation (lct_compress): wait for it only now, with the first source rows in flight.
-  cudaGridDependencySynchronize();
-  {
-    const uint32_t packed = (uint32_t)shifted_encode[tid];
-    // Clearing the payload image hides the latency of the table load.
-    for (int w = 0; w < g.fixed_words; ++w) payload[w * kLanes + tid] = 0u;
-    if (block == 0 && tid < 4) encoded[g.streams * g.fixed_words + tid] = 0u;  // trailing pad words
-    sh.table[tid] = make_uint2(packed & 0xFFFFFu, packed >> 20);
-  }
-  __syncthreads();
-
-  // Half tiles of 16 rows alternate between the two sides: the row side splits half tile h + 1
-  // into the free half of the warp's tile buffer (and ends by requesting the source of half
-  // tile h + 2, which then has a whole lane phase to arrive), the lanes encode half tile h.
-  // Issuing the row side's work between the lanes' lookups instead (one instruction stream)
-  // was measured slower: 66-68 us against 61.5 for 64 Mi elements.
-  rows.rest();   // half tile 0; leaves the source of half tile 1 requested
-  __syncwarp();
-  NoSlices nothing;
-  auto lanes = [&](auto half_tag, int h) {
-    constexpr int kHalf = decltype(half_tag)::value;
-    if (full_block)
-      encode_half_rows<false, kLaneMask, kHalf>(table_address, tile_lane, sink, g.lane_mask,
-                                                kTileRows * (h >> 1), valid, budget_bits, pos, lo,
-                                                extra_start, open, nothing);
-    else
-      encode_half_rows<true, kLaneMask, kHalf>(table_address, tile_lane, sink, g.lane_mask,
-                                               kTileRows * (h >> 1), valid, budget_bits, pos, lo,
-                                               extra_start, open, nothing);
-  };
-  for (int h = 0; h < halves; h += 2) {
-    lanes(std::integral_constant<int, 0>(), h);
-    __syncwarp();
-    if (h + 1 < halves) {
-      rows.rest();
-      __syncwarp();
-      lanes(std::integral_constant<int, 1>(), h + 1);
-      __syncwarp();
-      if (h + 2 < halves) {
-        rows.rest();
-        __syncwarp();
-      }
-    }
-  }
-  if (!kPrecomputed && !full_block) {
-    const int first_untouched = halves * (kTileRows / 2);
-    uint4* rest = reinterpret_cast<uint4*>(side + block_base + (int64_t)first_untouched * kLanes);
-    for (int i = tid; i < (g.steps - first_untouched) * (kLanes / 16); i += kThreads)
+  // Rows of this block that hold elements, in whole chunks.  Rows of pure padding (the tail of a
+  // ragged or tiny tensor) carry no bits; their side bytes are cleared in one sweep.
+  const int64_t left = g.logical_numel - block_base;
+  const int in_block = (int)max((int64_t)0, min((int64_t)g.block_symbols, left));
+  const int full_rows = in_block / kLanes;
+  const int rows_used = (in_block + kChunkRows * kLanes - 1) / (kChunkRows * kLanes) * kChunkRows;
+  BlockEncoder<kPrecomputed, kLaneMask> encoder{
+      static_cast<const char*>(src) + block_base * (kPrecomputed ? 1 : 2),
+      side + block_base + 2 * tid, g, block, 0u,
+      src_word_ok ? full_rows / kChunkRows * kChunkRows : 0, {}, {}};
+  // A full block of an aligned source is fetched ahead; the first portions now, with everything
+  // up to the table still to come.
+  const bool prefetches = !kPrecomputed && tid == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
+  if (prefetches && encoder.wide_rows >= kPrefetchRows)
+    prefetch_l2(encoder.rows, kPrefetchRows * kRowBytes);
+  clear_image(image, g.fixed_words);
+  if (block == 0 && tid < 4) encoded[g.streams * g.fixed_words + tid] = 0u;  // trailing pad words
+  if (!kPrecomputed && rows_used < g.steps) {
+    uint4* rest = reinterpret_cast<uint4*>(side + block_base + (int64_t)rows_used * kLanes);
+    for (int i = tid; i < (g.steps - rows_used) * (kLanes / 16); i += kPairThreads)
       __stcs(rest + i, make_uint4(0u, 0u, 0u, 0u));
   }
-  if (open && (pos & 31) != 0) payload_column[(pos >> 5) * kLanes] = lo;
-  extra_starts[block * kLanes + tid] = extra_start < 0 ? (uint8_t)255 : (uint8_t)extra_start;
+  // Everything above is independent of the tensor's center.  The shifted table may come from a
+  // kernel that is still running when this grid was launched with programmatic stream
+  // serialisation (lct_compress): wait for it only now.
+  cudaGridDependencySynchronize();
+  load_encode_table(sh.table, shifted_encode);
+  __syncthreads();
 
-  // Block summary: overflowing lanes and their tail bytes.
-  int bad = extra_start >= 0 ? 1 : 0;
-  int bytes = extra_start >= 0 ? g.steps - extra_start : 0;
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) {
-    bad += __shfl_down_sync(0xFFFFFFFFu, bad, d);
-    bytes += __shfl_down_sync(0xFFFFFFFFu, bytes, d);
-  }
-  if (lane32 == 0) { sh.scan[warp] = bad; sh.scan[8 + warp] = bytes; }
-  __syncthreads();  // also publishes every lane's payload words
-  if (tid == 0) {
-    int total_bad = 0, total_bytes = 0;
-    for (int w = 0; w < kWarps; ++w) { total_bad += sh.scan[w]; total_bytes += sh.scan[8 + w]; }
-    summaries[block] = total_bad;
-    summaries[g.n_blocks + block] = total_bytes;
-  }
-  // Payload image -> global: word w of the block's 256 streams is one 1 KB row.
-  uint32_t* out = encoded + block * kLanes;
-  for (int i = tid; i < g.fixed_words * (kLanes / 4); i += kThreads) {
-    const int w = i >> 6, c = (i & 63) * 4;
-    const uint4 v = *reinterpret_cast<const uint4*>(&payload[w * kLanes + c]);
-    __stcs(reinterpret_cast<uint4*>(out + (int64_t)w * g.streams + c), v);
-  }
+  encoder.a.open(shared_address(image + 2 * tid));
+  encoder.b.open(shared_address(image + 2 * tid + 1));
+  encoder.table = after_barrier(shared_address(sh.table));
+  encoder.run(rows_used, prefetches);
+  finish_block(encoder.a, encoder.b, image, sh.scan, encoded, extra_starts, summaries, block,
+               g.n_blocks, g.streams, g.steps, g.fixed_words);
 }
 
+// A closed lane must stay on the checked path: it closed within one pair (32 bits) of its budget.
+static_assert(kChunkBits >= 32, "a closed lane is near its budget");
+
 template <bool kPrecomputed, int kLaneMask>
-__global__ void __launch_bounds__(kThreads, kEncodeMinCtas)
-encode_kernel(const void* __restrict__ src, bool src_vector_ok, uint8_t* __restrict__ side,
-              uint32_t* __restrict__ encoded, const int32_t* __restrict__ shifted_encode,
+__global__ void __launch_bounds__(kPairThreads, kEncodeMinCtas)
+encode_kernel(const void* __restrict__ src, bool src_word_ok, uint8_t* __restrict__ side,
+              uint32_t* __restrict__ encoded, const int32_t* shifted_encode,
               uint8_t* __restrict__ extra_starts, int32_t* __restrict__ summaries, EncodeShape g) {
-  encode_block<kPrecomputed, kLaneMask>(src, src_vector_ok, side, encoded, shifted_encode,
+  encode_block<kPrecomputed, kLaneMask>(src, src_word_ok, side, encoded, shifted_encode,
                                         extra_starts, summaries, g, blockIdx.x);
 }
 
@@ -340,16 +281,16 @@ __device__ __forceinline__ int find_encode_job(const Job* jobs, int n_jobs, int6
 }
 
 template <int kLaneMask>
-__global__ void __launch_bounds__(kThreads, kEncodeMinCtas)
+__global__ void __launch_bounds__(kPairThreads, kEncodeMinCtas)
 encode_batch_kernel(const lct_encode_job* __restrict__ jobs, int n_jobs,
-                    const int32_t* __restrict__ shifted_encode, uint8_t* __restrict__ extra_starts,
+                    const int32_t* shifted_encode, uint8_t* __restrict__ extra_starts,
                     int32_t* __restrict__ summaries, EncodeShape common) {
   const int64_t block = blockIdx.x;
   const int j = find_encode_job(jobs, n_jobs, block);
   const lct_encode_job& job = jobs[j];
   const EncodeShape g = shape_of_job(job, common);
-  const bool vector_ok = (reinterpret_cast<uintptr_t>(job.src) & 15u) == 0;
-  encode_block<false, kLaneMask>(job.src, vector_ok, job.side,
+  const bool word_ok = (reinterpret_cast<uintptr_t>(job.src) & 3u) == 0;
+  encode_block<false, kLaneMask>(job.src, word_ok, job.side,
                                  reinterpret_cast<uint32_t*>(job.encoded),
                                  shifted_encode + 256 * (int64_t)j,
                                  extra_starts + job.first_block * kLanes,
@@ -361,12 +302,12 @@ encode_batch_kernel(const lct_encode_job* __restrict__ jobs, int n_jobs,
 // row from its overflow start to the end of the block (padding rows read as
 // exponent byte 0).
 template <bool kPrecomputed>
-__device__ __forceinline__ void compact_block(const void* __restrict__ src, uint8_t* lanes,
+__device__ __forceinline__ void compact_block(const void* src, uint8_t* lanes,
                                               uint8_t* starts, uint8_t* tail,
                                               const int32_t* descriptor, const int32_t* counts,
                                               int32_t* blocks_out,
-                                              const uint8_t* __restrict__ extra_starts,
-                                              const int32_t* __restrict__ summaries,
+                                              const uint8_t* extra_starts,
+                                              const int32_t* summaries,
                                               const EncodeShape& g, int64_t block) {
   __shared__ int scan[33];
   const int tid = threadIdx.x;
@@ -424,9 +365,9 @@ __device__ __forceinline__ void compact_block(const void* __restrict__ src, uint
 
 template <bool kPrecomputed>
 __global__ void __launch_bounds__(kThreads)
-compact_tails_kernel(const void* __restrict__ src, uint8_t* lanes, uint8_t* starts, uint8_t* tail,
+compact_tails_kernel(const void* src, uint8_t* lanes, uint8_t* starts, uint8_t* tail,
                      const int32_t* descriptor, const int32_t* counts, int32_t* blocks_out,
-                     const uint8_t* __restrict__ extra_starts, const int32_t* __restrict__ summaries,
+                     const uint8_t* extra_starts, const int32_t* summaries,
                      EncodeShape g) {
   cudaGridDependencySynchronize();  // prefixes and the reservation come from the scan in front
   compact_block<kPrecomputed>(src, lanes, starts, tail, descriptor, counts, blocks_out,
@@ -441,7 +382,7 @@ __device__ __forceinline__ const void* tail_source(const lct_update_job& job) { 
 template <typename Job, bool kPrecomputed>
 __global__ void __launch_bounds__(kThreads)
 compact_batch_kernel(const Job* __restrict__ jobs, int n_jobs, uint8_t* arena_payload,
-                     const uint8_t* __restrict__ extra_starts, const int32_t* __restrict__ summaries,
+                     const uint8_t* extra_starts, const int32_t* summaries,
                      EncodeShape common) {
   cudaGridDependencySynchronize();  // prefixes and reservations come from the scan in front
   const int64_t block = blockIdx.x;
@@ -494,7 +435,7 @@ static int launch_encode(const void* src, uint8_t* side, int32_t* encoded,
   if ((reinterpret_cast<uintptr_t>(encoded) & 15u) ||
       (!precomputed && (reinterpret_cast<uintptr_t>(side) & 15u)))
     return LCT_E_ALIGNMENT;
-  const bool vector_ok = (s & (precomputed ? 7u : 15u)) == 0;
+  const bool word_ok = (s & (precomputed ? 1u : 3u)) == 0;
   const size_t shared = sizeof(lct::EncodeSharedHead) + (size_t)fixed_words * lct::kLanes * 4;
   uint32_t* words = reinterpret_cast<uint32_t*>(encoded);
   const bool swizzled = g.lane_mask == 254;
@@ -503,9 +444,9 @@ static int launch_encode(const void* src, uint8_t* side, int32_t* encoded,
   rc = (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
   if (rc) return rc;
   if (overlapped)
-    return lct::launch_overlapped(kernel, (unsigned)g.n_blocks, lct::kThreads, shared, st, src,
-                                  vector_ok, side, words, shifted_encode, extra_starts, summaries, g);
-  kernel<<<(unsigned)g.n_blocks, lct::kThreads, shared, st>>>(src, vector_ok, side, words,
+    return lct::launch_overlapped(kernel, (unsigned)g.n_blocks, lct::kPairThreads, shared, st, src,
+                                  word_ok, side, words, shifted_encode, extra_starts, summaries, g);
+  kernel<<<(unsigned)g.n_blocks, lct::kPairThreads, shared, st>>>(src, word_ok, side, words,
                                                               shifted_encode, extra_starts,
                                                               summaries, g);
   return (int)cudaGetLastError();
@@ -633,7 +574,7 @@ int lct_compress_batch(const lct_encode_job* jobs, int n_jobs, int64_t total_blo
   if (rc) return rc;
   // Centers first (ordinary launch); the three kernels behind it may each be scheduled while
   // their predecessor still runs and wait for it on the device.
-  if ((rc = lct::launch_overlapped(encode_all, (unsigned)total_blocks, lct::kThreads,
+  if ((rc = lct::launch_overlapped(encode_all, (unsigned)total_blocks, lct::kPairThreads,
                                    shared, st, jobs, n_jobs, shifted_encode, extra_starts,
                                    summaries, g)))
     return rc;

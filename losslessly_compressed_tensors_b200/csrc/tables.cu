@@ -30,7 +30,7 @@ __device__ __forceinline__ void write_shifted_tables(const int32_t* __restrict__
 // sample loads together, and the base-table rows the shifted tables are made
 // from before the samples come back.
 template <bool kPrecomputed>
-__device__ __forceinline__ void center_and_tables(const void* __restrict__ src, int64_t n,
+__device__ __forceinline__ void center_and_tables(const void* src, int64_t n,
                                                   const int32_t* __restrict__ base_encode,
                                                   const int32_t* __restrict__ base_decode,
                                                   int32_t* center_out, int32_t* shifted_encode,
@@ -53,7 +53,7 @@ __device__ __forceinline__ void center_and_tables(const void* __restrict__ src, 
 
 template <bool kPrecomputed>
 __global__ void __launch_bounds__(kTableThreads)
-center_and_tables_kernel(const void* __restrict__ src, int64_t n,
+center_and_tables_kernel(const void* src, int64_t n,
                          const int32_t* __restrict__ base_encode,
                          const int32_t* __restrict__ base_decode, int32_t* center_out,
                          int32_t* shifted_encode, int32_t* shifted_decode) {
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(kTableThreads)
 center_update_batch_kernel(const lct_update_job* __restrict__ jobs,
                            const int32_t* __restrict__ base_encode,
                            const int32_t* __restrict__ base_decode,
-                           const uint8_t* __restrict__ samples, int32_t* shifted_encode) {
+                           const uint8_t* samples, int32_t* shifted_encode) {
   // The samples come from the kernel in front; the fused kernel behind may start its
   // table-independent prologue right away.
   cudaGridDependencySynchronize();

@@ -287,7 +287,7 @@ __device__ __forceinline__ void split_row(const uint32_t r[4], uint32_t q, uint3
 template <int kLaneMask, int kEmit>
 __device__ __forceinline__ void update_fused_block(
     const OperandView& a, const Shape& g_in, const uint16_t* other,
-    bool other_vector_ok, const OpSpec& spec, const int32_t* __restrict__ shifted_encode,
+    bool other_vector_ok, const OpSpec& spec, const int32_t* shifted_encode,
     uint8_t* __restrict__ side_out, uint32_t* __restrict__ encoded_out,
     uint8_t* __restrict__ extra_starts, int32_t* __restrict__ summaries,
     uint8_t* __restrict__ spill, uint16_t* dense_out, int64_t block) {
@@ -307,7 +307,7 @@ __device__ __forceinline__ void update_fused_block(
   // table (which may still be running when the grid was launched by lct_update).
   prepare_block(sh, a, g, block, [&] {
     cudaGridDependencySynchronize();
-    const uint32_t packed = (uint32_t)shifted_encode[tid];
+    const uint32_t packed = load_dependent_u32(shifted_encode + tid);
     encode_table[tid] = make_uint2(packed & 0xFFFFFu, packed >> 20);
   });  // ends with a block barrier
 
@@ -451,7 +451,7 @@ __device__ __forceinline__ void update_fused_block(
 template <int kLaneMask, int kEmit>
 __global__ void __launch_bounds__(kThreads, 4)
 update_fused_kernel(OperandView a, Shape g, const uint16_t* other, bool other_vector_ok,
-                    OpSpec spec, const int32_t* __restrict__ shifted_encode,
+                    OpSpec spec, const int32_t* shifted_encode,
                     uint8_t* __restrict__ side_out, uint32_t* __restrict__ encoded_out,
                     uint8_t* __restrict__ extra_starts, int32_t* __restrict__ summaries,
                     uint8_t* __restrict__ spill, uint16_t* dense_out) {
@@ -464,7 +464,7 @@ update_fused_kernel(OperandView a, Shape g, const uint16_t* other, bool other_ve
 template <int kLaneMask, int kEmit>
 __global__ void __launch_bounds__(kThreads, 4)
 update_fused_batch_kernel(const lct_update_job* __restrict__ jobs, int n_jobs, Shape common,
-                          OpSpec spec, const int32_t* __restrict__ shifted_encode,
+                          OpSpec spec, const int32_t* shifted_encode,
                           uint8_t* __restrict__ extra_starts, int32_t* __restrict__ summaries) {
   const int64_t block = blockIdx.x;
   int lo = 0, hi = n_jobs - 1;
