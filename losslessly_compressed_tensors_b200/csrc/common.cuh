@@ -40,15 +40,14 @@ constexpr int kSampleCount = 4096;     // positions the exponent center is estim
 
 // Two-symbol table entry (one per 12-bit stream window):
 //
-//   bits 0..4    bits to consume: both code lengths of a full pair (two directly coded
-//                symbols that fit the window together), else the first symbol's length
-//                (an escape: prefix + 8-bit literal).  A funnel shift takes its amount from
-//                the low five bits of a register, so the entry itself is the shift operand.
-//   bits 5..7    first code length - 1 of a full pair (for a reader that wants one symbol)
+//   byte 0       bits to consume: both code lengths of a full pair (two directly coded symbols
+//                that fit the window together), else the first symbol's length (an escape:
+//                prefix + 8-bit literal).  A funnel shift takes its amount from the low five
+//                bits of a register, so the entry itself is the shift operand, and one byte dot
+//                product subtracts the byte from a bit counter.
 //   byte 1       first symbol as an exponent byte (undefined for an escape)
 //   byte 2       second symbol of a full pair
-//   bits 24..28  copy of bits 0..4 for a full pair, else 0: one byte dot product subtracts it
-//                from a bit counter
+//   bits 24..28  first symbol's length (for a reader that wants one symbol)
 //   bit 30       kEscape: the first symbol is an escape
 //   bit 31       kSlow: not a full pair (the sign bit, so one signed compare finds it)
 constexpr uint32_t kSlow = 0x80000000u;
@@ -56,17 +55,15 @@ constexpr uint32_t kEscape = 0x40000000u;
 
 __host__ __device__ __forceinline__ uint32_t make_pair_entry(uint32_t len0, uint32_t byte0,
                                                              uint32_t len1, uint32_t byte1) {
-  const uint32_t total = len0 + len1;
-  return total | ((len0 - 1u) << 5) | (byte0 << 8) | (byte1 << 16) | (total << 24);
+  return (len0 + len1) | (byte0 << 8) | (byte1 << 16) | (len0 << 24);
 }
+// A first symbol's length is at most 16 (a prefix of 8 and an 8-bit literal).
 __host__ __device__ __forceinline__ uint32_t make_single_entry(uint32_t len0, uint32_t byte0,
                                                                bool escape) {
-  return kSlow | (escape ? kEscape : 0u) | len0 | (byte0 << 8);
+  return kSlow | (escape ? kEscape : 0u) | (len0 & 31u) | (byte0 << 8) | ((len0 & 31u) << 24);
 }
 // Length of the entry's first symbol.
-__device__ __forceinline__ uint32_t entry_first_length(uint32_t entry) {
-  return (int32_t)entry < 0 ? (entry & 31u) : ((entry >> 5) & 7u) + 1u;
-}
+__device__ __forceinline__ uint32_t entry_first_length(uint32_t entry) { return (entry >> 24) & 31u; }
 __device__ __forceinline__ uint32_t entry_first_symbol(uint32_t entry) { return (entry >> 8) & 255u; }
 __device__ __forceinline__ uint32_t entry_second_symbol(uint32_t entry) { return (entry >> 16) & 255u; }
 

@@ -1,29 +1,27 @@
 // Table-driven decoder and the fused decode -> pointwise operation kernels.
 //
-// One CTA (256 threads) per codec block.
+// One CTA of 256 threads per codec block, thread = lane (lanes.cuh, lane_reader.cuh).
 //
-// Prologue: the block's payload tile (fixed_words rows of 256 words) and the
-// 16 KB two-symbol table of this tensor's center are copied into shared memory
-// with cp.async while the block's overflow map is expanded.
+// Prologue: the block's payload and the 16 KB two-symbol table of this tensor's center are copied
+// into shared memory with cp.async while the block's overflow map is expanded.
 //
-// Then, software pipelined over half tiles of 16 rows:
-//   lane side - thread = lane: the next 94 bits of its stream in three registers,
-//               pre-shifted so that 12 of them index the two-symbol table (two
-//               exponent bytes + bits consumed per lookup); consuming is three
-//               funnel shifts by the table entry itself, refills from the shared
-//               image are off the lookup chain (decode_core.cuh: ShiftCursor).
-//               The only divergent path is the rare entry that is not a full
-//               pair, decoded one symbol at a time;
-//   row side  - thread = 8 columns of a row pair of the PREVIOUS half tile:
-//               128-bit read of the tile, 64-bit side-byte loads (requested a
-//               half tile earlier), four bytes at a time rebuilt into BF16,
-//               optional arithmetic, 128-bit streaming stores.  In the plain
-//               decoder its instructions are issued between the lane side's
-//               lookups, and two neighbouring warps share their rows out so
-//               that every store instruction writes full 128-byte lines.
-// Overflow lanes switch from the bit stream to their raw tail bytes at their
-// recorded start step, inside the same launch.
-#include "decode_core.cuh"
+// Then, per row pair: one table lookup gives a lane's two exponents and the bits to consume (two
+// funnel shifts by the table entry itself); one shuffle gives every thread both columns' exponents
+// of one row; these are joined with two side bytes out of the warp's ring to one word of the dense
+// tensor.  The stores of a pair are issued while the next pair's lookup is under way.  The only
+// divergent path is the rare entry that is not a full pair.
+//
+// Bound by instruction issue (75 % of the issue slots, 45 instructions per warp and pair at 64 Mi
+// weights, a quarter of them the not-a-full-pair path).  Against the former form (16-row tiles
+// transposed through shared memory to eight columns per thread, 50 instructions), at 64 Mi
+// elements: 69.0 -> 59.3 us (weights with outliers), 58.8 -> 52.1 (normal), 60.6 -> 52.8 (half
+// zeros, overflow); 1 Mi: 11.3 -> 9.4.  Measured and left: two lanes per thread (90 us: half the
+// warps, each with twice the serial chain), side bytes requested into registers (90 us: the loads'
+// registers spill, which waits for every load at once), 3 instead of 4 CTAs per SM (61.0).
+//
+// Overflow lanes switch from the bit stream to their raw tail bytes at their recorded start step,
+// inside the same launch.
+#include "lane_reader.cuh"
 
 namespace lct {
 
@@ -31,138 +29,71 @@ namespace lct {
 // Plain decode
 // ---------------------------------------------------------------------------
 
+// One codec block: 256 threads, thread = lane.  Per row pair a thread looks up one table entry of
+// its lane - two symbols - exchanges exponents with its neighbour, joins those of its row with the
+// side bytes of the two columns and stores one word.  Side bytes come through a ring in shared memory.
 // kLaneMask: the lane mapping as a compile-time constant (254, the default mapping: the masked
-// tile and row addresses fold into constants, 80 instead of 82 us per 64 Mi elements), or -1 to
-// take it from the shape at run time (the linear mapping).
-// Row side of one half tile (16 rows) for one thread: 8 columns of one row pair.  Cut into
-// slices that the lane phase of the NEXT half tile issues between its pairs.
-struct DecodeRowSlices {
-  const uint16_t* tile;
-  uint16_t* out;
-  SideSelectors selectors;
-  int64_t logical_numel;
-  bool full_block;
-  // the half tile being finished:
-  UnitPlace place;
-  uint2 side[2];
-  uint4 words;
-  uint32_t top[4], bottom[4];
+// row addresses fold into constants), or -1 to take it from the shape at run time.
+template <int kLaneMask>
+struct BlockDecoder {
+  const Shape& g;
+  int64_t row0;
+  DenseWords<uint16_t> out;
+  RowExchange rows;
+  SideRing sides;
+  LaneWalk walk;
 
-  __device__ __forceinline__ void store(const uint32_t (&row)[4], int64_t at) {
-    if (full_block || at + 8 <= logical_numel) {
-      __stcs(reinterpret_cast<uint4*>(out + at), make_uint4(row[0], row[1], row[2], row[3]));
-    } else {
+  __device__ __forceinline__ void chunk(int step0) {
+    const uint32_t offset = word_offset(row0, step0, g.lane_mask);
+    if (walk.whole_chunk(step0)) {
+      uint32_t entry = 0u, neighbour = 0u, side = 0u;
+      auto emit = [&](int k) {
+        out.store(word_at<kLaneMask>(offset, k, g.lane_mask),
+                  join_word(rows.exponents(entry, neighbour), side));
+      };
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (at + i < logical_numel) out[at + i] = (uint16_t)(row[i >> 1] >> (16 * (i & 1)));
+      for (int k = 0; k < kWalkPairs; ++k) {
+        entry = walk.read_pair(k, [&] { if (k > 0) emit(k - 1); });
+        neighbour = rows.neighbours(entry);
+        side = sides.pair(k);
+      }
+      emit(kWalkPairs - 1);
+    } else {
+      walk.read_chunk(step0, g.steps, [&](int k, uint32_t entry) {
+        out.store_guarded(word_at<kLaneMask>(offset, k, g.lane_mask),
+                          join_word(rows.exponents(entry, rows.neighbours(entry)), sides.pair(k)));
+      });
     }
-  }
-  template <int k>
-  __device__ __forceinline__ void slice() {
-    if (k == 0) words = *reinterpret_cast<const uint4*>(&tile[place.tile_index]);
-    if (k == 1) join_row(words, side[0], selectors, false, top);
-    if (k == 2) store(top, place.logical);
-    if (k == 3) join_row(words, side[1], selectors, true, bottom);
-    if (k == 4) store(bottom, place.logical + kLanes);
-  }
-  __device__ __forceinline__ void rest() {
-    slice<0>(); slice<1>(); slice<2>(); slice<3>(); slice<4>();
   }
 };
 
-// One codec block.  The work is software pipelined over half tiles of 16 rows: while a warp's
-// lanes decode half tile h into one half of the warp's tile buffer, the row side of half tile
-// h - 1 (join with the side bytes, 128-bit stores) is issued between the lookups from the other
-// half of the buffer, and the side bytes of half tile h were requested one iteration earlier.
-// kLaneMask: the lane mapping as a compile-time constant (254, the default mapping), or -1 to
-// take it from the shape at run time (the linear mapping).
 template <int kLaneMask>
 __device__ __forceinline__ void decode_block(const OperandView& a, const Shape& g_in,
                                              uint16_t* __restrict__ out, int64_t block) {
   Shape g = g_in;
   if (kLaneMask >= 0) g.lane_mask = kLaneMask;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane32 = tid & 31;
-  const int64_t row0 = block * g.steps;
   const int64_t block_base = block * (int64_t)g.block_symbols;
-  const OperandShared sh = carve_operand(smem_raw, 0, 1, g.fixed_words);
-  prepare_block(sh, a, g, block);
-
-  const int valid = valid_steps_of(block, tid, g.steps, g.block_symbols, g.logical_numel, g.lane_mask);
-  LaneState lane = open_lane(sh, a, g, valid);
-  const bool full_block = block_base + g.block_symbols <= g.logical_numel;
-  // Rows of this block that hold elements: half tiles of pure padding (the tail of a ragged or
-  // tiny tensor) have nothing to decode and nothing to store.
-  const int rows_used =
-      full_block ? g.steps : (int)((g.logical_numel - block_base + kLanes - 1) / kLanes);
-  const int halves = (rows_used + kTileRows / 2 - 1) / (kTileRows / 2);
-
-  // Row side: kRowWarps neighbouring warps work as one group.  Their lanes cover one aligned
-  // segment of 32 * kRowWarps columns in every row (the lane mapping's bits 5..7 move whole
-  // aligned groups), and the group's threads share that segment out so that 4 * kRowWarps
-  // neighbouring threads cover one row: 128-bit stores of full 128-byte lines from two warps on.
-  constexpr int kRowWarps = 2, kRowShift = 1;  // measured: 1 -> 76.8 us, 2 -> 75.9, 4 -> 78.0 (64 Mi elements)
-  const int group = warp >> kRowShift;
-  const int in_group = ((warp & (kRowWarps - 1)) << 5) + lane32;
-  const int column8 = in_group & (4 * kRowWarps - 1);  // which 8 columns of the segment
-  const int pair8 = in_group >> (2 + kRowShift);        // which row pair of a half tile, 0..7
-  auto group_barrier = [&] {
-    if (kRowWarps == 1) __syncwarp();
-    else asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(32 * kRowWarps) : "memory");
-  };
-
-  DecodeRowSlices rows;
-  rows.out = out;
-  // Every row-side unit of a thread has the same pair permutation (its pair index mod 4).
-  rows.selectors = side_selectors((uint32_t)(((2 * pair8) & g.lane_mask) >> 1) & 3u);
-  rows.logical_numel = g.logical_numel;
-  rows.full_block = full_block;
-
-  // Side bytes of half tile h for this thread's unit (row pair 8 * (h & 1) + pair8 of tile h / 2).
-  UnitPlace next_place;
-  const uint16_t* next_tile;
-  uint2 next_side[2];
-  auto request = [&](int h) {
-    const int step0 = kTileRows * (h >> 1);
-    // The warp of the group whose lanes hold these columns in this tile.
-    const int moved = (int)((row0 + step0) & g.lane_mask) >> 5;
-    const int owner = (group << kRowShift) + ((column8 >> 2) ^ (moved & (kRowWarps - 1)));
-    next_place = place_unit(owner, kHalfPairs * (h & 1) + pair8, column8 & 3, row0, step0,
-                            block_base, g.lane_mask);
-    next_tile = sh.head->tile[owner];
-    const uint8_t* s = a.side + next_place.storage;
-    next_side[0] = __ldcs(reinterpret_cast<const uint2*>(s));
-    next_side[1] = __ldcs(reinterpret_cast<const uint2*>(s + kLanes));
-  };
-  auto hand_over = [&] {
-    rows.place = next_place;
-    rows.tile = next_tile;
-    rows.side[0] = next_side[0];
-    rows.side[1] = next_side[1];
-  };
-  NoSlices nothing;
-  request(0);
-  // Half tile 0: nothing to finish yet.
-  decode_half_rows<kLaneMask, 0>(lane.reader, lane.tables, 0, lane.coded, lane.tail_from,
-                                 lane.tail_bytes, g.rare_length, g.lane_mask, nothing);
-  hand_over();
-  group_barrier();
-  // One copy of the code serves both halves of the tile buffer (the second half's rows are
-  // 512 bytes further on): the loop stays within the instruction cache.
-  LaneTables tables = lane.tables;
+  const ReaderShared sh = carve_reader(smem_raw, 0, 1, g.fixed_words, kRingBytes);
+  // Rows of pure padding (the tail of a ragged or tiny tensor) have nothing to decode or store.
+  const int rows_used = rows_in_use(g, block);
+  BlockDecoder<kLaneMask> decoder{g, block * g.steps, {out + block_base, g.logical_numel - block_base},
+                                  {}, {}, {}};
+  decoder.sides.open(smem_raw + kTableBytes, a.side + block_base, rows_used);
+  stage_operand(sh, a, g, block);
+  decoder.rows.open();
+  cp_async_wait_all();
+  __syncthreads();
+  decoder.walk.open(sh, a, g, block);
 #pragma unroll 1
-  for (int h = 1; h < halves; ++h) {
-    request(h);
-    tables.tile_lane = lane.tables.tile_lane + (uint32_t)((h & 1) * kHalfPairs * 64);
-    decode_half_rows<kLaneMask, 0>(lane.reader, tables, (kTileRows / 2) * h, lane.coded,
-                                   lane.tail_from, lane.tail_bytes, g.rare_length, g.lane_mask, rows);
-    hand_over();
-    group_barrier();
+  for (int step0 = 0; step0 < rows_used; step0 += kWalkRows) {
+    decoder.sides.wait();
+    decoder.chunk(step0);
+    decoder.sides.advance();
   }
-  rows.rest();  // the last half tile
 }
 
-// Resident CTAs per SM the decoder is compiled for (shared memory allows no more; three cost 8 %).
+// Resident CTAs per SM the decoder is compiled for.
 constexpr int kDecodeMinCtas = 4;
 template <int kLaneMask>
 __global__ void __launch_bounds__(kThreads, kDecodeMinCtas)
@@ -240,85 +171,152 @@ decode_batch_kernel(const lct_decode_job* __restrict__ jobs, int n_jobs, Shape c
 // Fused pointwise operations
 // ---------------------------------------------------------------------------
 
+// One codec block, divided among threads as in the plain decoder.  The second operand is a dense
+// tensor (its words are requested ahead, like the side bytes) or, kDual, another compressed one,
+// whose lane the same thread walks.
+// `compressed`: the result leaves as side bytes (storage order) and exponent bytes (`auxiliary`,
+// element order) instead of dense values; padding counts as +0.0.
+// Measured against the former tile form: 3072 x 4096 one compressed operand 41.0 -> 35.2 us, two
+// compressed operands and a compressed result (768 x 2304) 46.8 -> 35.8; 8192 x 4096 in blocks of
+// 32768 54.8 -> 56.9 (the one size found that lost).
 template <bool kDual, int kLaneMask>
-__global__ void __launch_bounds__(kThreads)
-pointwise_kernel(OperandView a, OperandView b, Shape g_in, const uint16_t* __restrict__ other,
-                 bool other_vector_ok, void* output, uint8_t* auxiliary, OpSpec spec,
+struct BlockPointwise {
+  const Shape& g;
+  Operation operation;
+  int64_t row0;
+  DenseWords<const uint16_t> other;
+  int wide_rows;  // rows, in whole chunks, of `other` that may be read as words
+  bool compressed;
+  DenseWords<uint16_t> out;  // dense result
+  uint8_t* side_out;
+  DenseWords<uint8_t> exponents_out;
+  int rows_used;
+  RowExchange rows;
+  SideRing sides_a, sides_b;
+  LaneWalk walk_a, walk_b;
+
+  using Buffer = uint32_t[kWalkPairs];
+  __device__ __forceinline__ void request(Buffer& words, int step0) const {
+    if (kDual || step0 >= rows_used) return;
+    const uint32_t offset = word_offset(row0, step0, g.lane_mask);
+#pragma unroll
+    for (int k = 0; k < kWalkPairs; ++k) {
+      const uint32_t at = word_at<kLaneMask>(offset, k, g.lane_mask);
+      words[k] = step0 < wide_rows ? other.load(at) : other.load_guarded(at);
+    }
+  }
+  __device__ __forceinline__ void emit(int step, uint32_t at, bool guarded, uint32_t exponents_a,
+                                       uint32_t exponents_b, uint32_t from_a, uint32_t from_b) const {
+    const uint32_t left = join_word(exponents_a, from_a);
+    const uint32_t right = kDual ? join_word(exponents_b, from_b) : from_b;
+    uint32_t result = operation(left, right);
+    if (!compressed) {
+      if (guarded) out.store_guarded(at, result);
+      else out.store(at, result);
+      return;
+    }
+    if (guarded) {
+      if ((int64_t)at >= out.left) result = 0u;
+      else if ((int64_t)at + 1 >= out.left) result &= 0xFFFFu;
+    }
+    uint32_t sides, exponents;
+    split_words(result, 0u, &sides, &exponents);
+    *reinterpret_cast<uint16_t*>(side_out + step * kLanes) = (uint16_t)sides;
+    if (guarded)
+      exponents_out.store_guarded(at, (exponents & 255u) | ((exponents & 0xFF00u) << 8));
+    else
+      *reinterpret_cast<uint16_t*>(exponents_out.rows + at) = (uint16_t)exponents;
+  }
+  __device__ __forceinline__ void chunk(int step0, Buffer& words) {
+    bool whole = walk_a.whole_chunk(step0);
+    if constexpr (kDual) whole = walk_b.whole_chunk(step0) && whole;
+    const uint32_t offset = word_offset(row0, step0, g.lane_mask);
+    if (whole) {
+      uint32_t entry_a = 0u, entry_b = 0u, neighbour_a = 0u, neighbour_b = 0u, side_a = 0u, side_b = 0u;
+      auto emit_pair = [&](int k) {
+        emit(step0 + 2 * k, word_at<kLaneMask>(offset, k, g.lane_mask), false,
+             rows.exponents(entry_a, neighbour_a), rows.exponents(entry_b, neighbour_b), side_a,
+             kDual ? side_b : words[k]);
+      };
+#pragma unroll
+      for (int k = 0; k < kWalkPairs; ++k) {
+        const uint32_t next_a = walk_a.read_pair(k, [&] { if (k > 0) emit_pair(k - 1); });
+        entry_a = next_a;
+        neighbour_a = rows.neighbours(entry_a);
+        side_a = sides_a.pair(k);
+        if constexpr (kDual) {
+          entry_b = walk_b.read_pair(k, [] {});
+          neighbour_b = rows.neighbours(entry_b);
+          side_b = sides_b.pair(k);
+        }
+      }
+      emit_pair(kWalkPairs - 1);
+    } else {
+      walk_a.read_chunk(step0, g.steps, [&](int k, uint32_t entry_a) {
+        const int step = step0 + 2 * k;
+        uint32_t entry_b = 0u;
+        if constexpr (kDual) entry_b = walk_b.read_any(step, walk_b.tail_pair(step, g.steps));
+        emit(step, word_at<kLaneMask>(offset, k, g.lane_mask), true,
+             rows.exponents(entry_a, rows.neighbours(entry_a)),
+             kDual ? rows.exponents(entry_b, rows.neighbours(entry_b)) : 0u, sides_a.pair(k),
+             kDual ? sides_b.pair(k) : words[0]);
+        if (!kDual) next_pair(words);
+      });
+    }
+  }
+};
+
+constexpr int kPointwiseMinCtas = 3, kDualMinCtas = 2;
+
+template <bool kDual, int kLaneMask>
+__global__ void __launch_bounds__(kThreads, kDual ? kDualMinCtas : kPointwiseMinCtas)
+pointwise_kernel(OperandView a, OperandView b, Shape g_in, const uint16_t* other,
+                 bool other_word_ok, void* output, uint8_t* auxiliary, OpSpec spec,
                  bool compressed) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Shape g = g_in;
-  if (kLaneMask >= 0) g.lane_mask = kLaneMask;  // see decode_block
-  const OperandShared sh = carve_operand(smem_raw, 0, kDual ? 2 : 1, g.fixed_words);
-  const OperandShared sh_b = carve_operand(smem_raw, kDual ? 1 : 0, kDual ? 2 : 1, g.fixed_words);
+  if (kLaneMask >= 0) g.lane_mask = kLaneMask;  // see BlockDecoder
+  constexpr int kOperands = kDual ? 2 : 1;
+  const ReaderShared sh = carve_reader(smem_raw, 0, kOperands, g.fixed_words, kOperands * kRingBytes);
+  const ReaderShared sh_b =
+      carve_reader(smem_raw, kOperands - 1, kOperands, g.fixed_words, kOperands * kRingBytes);
+  unsigned char* rings = smem_raw + kOperands * kTableBytes;
   const int64_t block = blockIdx.x;
-  const int tid = threadIdx.x, warp = tid >> 5, lane32 = tid & 31;
-  const int64_t row0 = block * g.steps;
+  const int tid = threadIdx.x;
   const int64_t block_base = block * (int64_t)g.block_symbols;
-  prepare_block(sh, a, g, block);
-  if (kDual) prepare_block(sh_b, b, g, block);
-
-  const float alpha = spec.alpha_is_one ? 1.0f : *spec.alpha;
-  const float beta = spec.beta_is_one ? 1.0f : *spec.beta;
-  const int valid = valid_steps_of(block, tid, g.steps, g.block_symbols, g.logical_numel, g.lane_mask);
-  LaneState lane_a = open_lane(sh, a, g, valid);
-  LaneState lane_b = lane_a;
-  if (kDual) lane_b = open_lane(sh_b, b, g, valid);
-  const uint16_t* tile = sh.head->tile[warp];
-  const uint16_t* tile_b = sh_b.head->tile[warp];
-  const SideSelectors selectors = side_selectors((uint32_t)(((2 * (lane32 >> 2)) & g.lane_mask) >> 1) & 3u);
-
-  for (int step0 = 0; step0 < g.steps; step0 += kTileRows) {
-    decode_tile_rows<kLaneMask>(lane_a.reader, lane_a.tables, step0, lane_a.coded, lane_a.tail_from,
-                                lane_a.tail_bytes, g.rare_length, g.lane_mask);
-    if (kDual)
-      decode_tile_rows<kLaneMask>(lane_b.reader, lane_b.tables, step0, lane_b.coded,
-                                  lane_b.tail_from, lane_b.tail_bytes, g.rare_length, g.lane_mask);
-    __syncwarp();
-    // All global loads of the tile's four rows first, so their latencies overlap.
-    UnitPlace place_of[2];
-    uint2 side_a[2][2], side_b[2][2];
-    uint32_t dense_in[2][2][4];
+  const int64_t left = g.logical_numel - block_base;
+  const int rows_used = rows_in_use(g, block);
+  uint8_t* side_out = static_cast<uint8_t*>(output) + block_base;
+  BlockPointwise<kDual, kLaneMask> work{
+      g, Operation(spec), block * g.steps, {other + (kDual ? 0 : block_base), left},
+      other_word_ok ? (int)min((int64_t)g.steps, left / kLanes) / kWalkRows * kWalkRows : 0, compressed,
+      {static_cast<uint16_t*>(output) + (compressed ? 0 : block_base), left},
+      side_out + own_bytes(), {auxiliary + (compressed ? block_base : 0), left}, rows_used, {}, {}, {},
+      {}, {}};
+  typename BlockPointwise<kDual, kLaneMask>::Buffer now, next;
+  work.request(now, 0);
+  if (kDual) work.sides_b.open(rings + kRingBytes, b.side + block_base, rows_used);
+  work.sides_a.open(rings, a.side + block_base, rows_used);
+  stage_operand(sh, a, g, block);
+  if (kDual) stage_operand(sh_b, b, g, block);
+  if (compressed)
+    for (int row = rows_used + (tid >> 6); row < g.steps; row += 4)
+      reinterpret_cast<uint32_t*>(side_out + row * kLanes)[tid & 63] = 0u;
+  work.rows.open();
+  cp_async_wait_all();
+  __syncthreads();
+  work.walk_a.open(sh, a, g, block);
+  if (kDual) work.walk_b.open(sh_b, b, g, block);
+#pragma unroll 1
+  for (int step0 = 0; step0 < rows_used; step0 += kWalkRows) {
+    work.request(next, step0 + kWalkRows);
+    if (kDual) work.sides_b.wait_both(work.sides_a);
+    else work.sides_a.wait();
+    work.chunk(step0, now);
+    work.sides_a.advance();
+    if (kDual) work.sides_b.advance();
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      place_of[u] = place_unit(warp, (lane32 >> 2) + 8 * u, lane32 & 3, row0, step0, block_base,
-                               g.lane_mask);
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int64_t s_at = place_of[u].storage + half * kLanes;
-        side_a[u][half] = __ldcs(reinterpret_cast<const uint2*>(a.side + s_at));
-        if (kDual)
-          side_b[u][half] = __ldcs(reinterpret_cast<const uint2*>(b.side + s_at));
-        else
-          load_dense8(other, place_of[u].logical + half * kLanes, g.logical_numel, other_vector_ok,
-                      dense_in[u][half]);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const UnitPlace place = place_of[u];
-      const uint4 words = *reinterpret_cast<const uint4*>(&tile[place.tile_index]);
-      uint4 words_b = make_uint4(0, 0, 0, 0);
-      if (kDual) words_b = *reinterpret_cast<const uint4*>(&tile_b[place.tile_index]);
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int64_t s_at = place.storage + half * kLanes;
-        const int64_t l_at = place.logical + half * kLanes;
-        uint32_t left[4], right[4], result[4];
-        join_row(words, side_a[u][half], selectors, half == 1, left);
-        if (kDual) {
-          join_row(words_b, side_b[u][half], selectors, half == 1, right);
-        } else {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) right[k] = dense_in[u][half][k];
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          result[k] = apply_op(left[k], right[k], spec.op, spec.alpha_is_one != 0,
-                               spec.beta_is_one != 0, alpha, beta);
-        store_row(result, compressed, output, auxiliary, l_at, g.logical_numel, s_at, place.q);
-      }
-    }
-    __syncwarp();
+    for (int k = 0; k < kWalkPairs; ++k) now[k] = next[k];
   }
 }
 
@@ -335,7 +333,7 @@ int lct_decode(const lct_operand* a, int16_t* out, int64_t size, int64_t logical
   if ((rc = lct::view_of(a, &va)) != 0) return rc;
   if (out == nullptr) return LCT_E_NULL_POINTER;
   if (!lct::aligned16(out)) return LCT_E_ALIGNMENT;
-  const size_t shared = lct::operand_shared_bytes(fixed_words);
+  const size_t shared = lct::reader_shared_bytes(1, fixed_words, lct::kRingBytes);
   auto kernel = g.lane_mask == 254 ? lct::decode_kernel<254> : lct::decode_kernel<-1>;
   if ((rc = lct::opt_in_shared(kernel, shared)) != 0) return rc;
   kernel<<<(unsigned)g.n_blocks, lct::kThreads, shared, static_cast<cudaStream_t>(stream)>>>(
@@ -351,7 +349,7 @@ int lct_decode_batch(const lct_decode_job* jobs, int n_jobs, int64_t total_block
   int rc = lct::check_shape(block_symbols, block_symbols, block_symbols, steps, fixed_words,
                             rare_length, &g);
   if (rc) return rc;
-  const size_t shared = lct::operand_shared_bytes(fixed_words);
+  const size_t shared = lct::reader_shared_bytes(1, fixed_words, lct::kRingBytes);
   auto kernel = g.lane_mask == 254 ? lct::decode_batch_kernel<254> : lct::decode_batch_kernel<-1>;
   if ((rc = lct::opt_in_shared(kernel, shared)) != 0) return rc;
   kernel<<<(unsigned)total_blocks, lct::kThreads, shared, static_cast<cudaStream_t>(stream)>>>(
@@ -375,11 +373,11 @@ int lct_pointwise(const lct_operand* a, const void* other, void* output, uint8_t
     return LCT_E_ALIGNMENT;
   if ((reinterpret_cast<uintptr_t>(other) & 1u) != 0) return LCT_E_ALIGNMENT;
   const lct::OpSpec spec{alpha, beta, op, alpha_is_one, beta_is_one};
-  const size_t shared = lct::operand_shared_bytes(fixed_words);
+  const size_t shared = lct::reader_shared_bytes(1, fixed_words, lct::kRingBytes);
   auto kernel = g.lane_mask == 254 ? lct::pointwise_kernel<false, 254> : lct::pointwise_kernel<false, -1>;
   if ((rc = lct::opt_in_shared(kernel, shared)) != 0) return rc;
   kernel<<<(unsigned)g.n_blocks, lct::kThreads, shared, static_cast<cudaStream_t>(stream)>>>(
-      va, va, g, static_cast<const uint16_t*>(other), lct::aligned16(other), output, auxiliary,
+      va, va, g, static_cast<const uint16_t*>(other), (reinterpret_cast<uintptr_t>(other) & 3u) == 0, output, auxiliary,
       spec, compressed_output != 0);
   return (int)cudaGetLastError();
 }
@@ -400,10 +398,10 @@ int lct_dual_scale_add(const lct_operand* a, const lct_operand* b, void* output,
     return LCT_E_ALIGNMENT;
   // fma(a, alpha, b): the scaled operation with beta == 1.
   const lct::OpSpec spec{alpha, nullptr, LCT_OP_SCALAR_MUL_ADD, 0, 1};
-  const size_t one = lct::operand_shared_bytes(fixed_words);
+  const size_t shared = lct::reader_shared_bytes(2, fixed_words, 2 * lct::kRingBytes);
   auto kernel = g.lane_mask == 254 ? lct::pointwise_kernel<true, 254> : lct::pointwise_kernel<true, -1>;
-  if ((rc = lct::opt_in_shared(kernel, 2 * one)) != 0) return rc;
-  kernel<<<(unsigned)g.n_blocks, lct::kThreads, 2 * one, static_cast<cudaStream_t>(stream)>>>(
+  if ((rc = lct::opt_in_shared(kernel, shared)) != 0) return rc;
+  kernel<<<(unsigned)g.n_blocks, lct::kThreads, shared, static_cast<cudaStream_t>(stream)>>>(
       va, vb, g, nullptr, false, output, auxiliary, spec, compressed_output != 0);
   return (int)cudaGetLastError();
 }

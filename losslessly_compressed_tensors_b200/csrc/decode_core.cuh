@@ -5,37 +5,10 @@
 // of the fused operations, and the host-side argument checks.
 #pragma once
 
-#include "common.cuh"
-#include "lct_b200.h"
+#include "lanes.cuh"
+#include "operand.cuh"
 
 namespace lct {
-
-struct OperandView {
-  const uint32_t* encoded;
-  const uint8_t* side;
-  const int32_t* center;
-  const uint32_t* pair_table;
-  const uint8_t* lanes;
-  const uint8_t* starts;
-  const uint8_t* tail;
-  const int32_t* descriptor;
-  const int32_t* count;
-  const int32_t* blocks;
-  int64_t base;
-  int mode;
-};
-
-struct Shape {
-  int64_t size;
-  int64_t logical_numel;
-  int64_t streams;
-  int64_t n_blocks;
-  int block_symbols;
-  int steps;
-  int fixed_words;
-  int rare_length;
-  int lane_mask;  // 254: lane ^ (row & 254) ("swizzle"); 0: "linear"
-};
 
 // Shared memory of a decoding CTA with n operands (n = 2 only for the fused operation on two
 // compressed tensors):
@@ -63,7 +36,6 @@ struct __align__(16) DecodeHead {
   int scan[36];
 };
 constexpr size_t kHeadBytes = 10240;
-constexpr size_t kTableBytes = (size_t)kPairEntries * 4;
 static_assert(sizeof(DecodeHead) <= kHeadBytes, "head must fit its slot");
 static_assert(kHeadBytes % 1024 == 0 && kHeadBytes >= 9 * 1024,
               "a lane may fetch up to 9 rows past the image");
@@ -95,35 +67,14 @@ __device__ __forceinline__ OperandShared carve_operand(unsigned char* base, int 
   return s;
 }
 
-__device__ __forceinline__ void cp_async_16(void* shared_dst, const void* global_src) {
-  const uint32_t dst = (uint32_t)__cvta_generic_to_shared(shared_dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(global_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_4(void* shared_dst, const void* global_src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
-                   (uint32_t)__cvta_generic_to_shared(shared_dst)),
-               "l"(global_src));
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-}
-
 // ---- shared memory by 32-bit address (lane phases) -------------------------
 // The lane phases address shared memory with 32-bit window addresses and constant
 // byte offsets, so that a lookup is one load with an immediate and no 64-bit
 // pointer arithmetic.
-__device__ __forceinline__ uint32_t shared_address(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
 template <int kByteOffset = 0>
 __device__ __forceinline__ uint32_t load_shared_u32(uint32_t address) {
   uint32_t v;
   asm volatile("ld.shared.u32 %0, [%1+%2];" : "=r"(v) : "r"(address), "n"(kByteOffset));
-  return v;
-}
-__device__ __forceinline__ uint32_t load_shared_u8(uint32_t address) {
-  uint32_t v;
-  asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(address));
   return v;
 }
 template <int kByteOffset = 0>
@@ -145,14 +96,6 @@ __device__ __forceinline__ void store_shared_u16_at(uint32_t address, uint32_t v
 __device__ __forceinline__ uint32_t funnel_right(uint32_t low, uint32_t high, uint32_t amount) {
   return __funnelshift_r(low, high, amount);  // the amount is taken modulo 32
 }
-// a + sum over the four bytes of e (unsigned) * w (signed): with w = -1 in one byte this
-// subtracts that byte of e from a.
-__device__ __forceinline__ int dot_bytes(uint32_t e, int w, int a) {
-  int d;
-  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(e), "r"(w), "r"(a));
-  return d;
-}
-
 // Shared address of the table entry for the window at bits 2..13 of `bits4` (the two low bits
 // are ignored).  The tables sit at fixed offsets of the CTA's shared memory, so `table` is a
 // constant that folds into the load's immediate.
@@ -209,7 +152,7 @@ struct ShiftCursor {
   // Consume a full-pair entry (refill separately).
   __device__ __forceinline__ void take_pair(uint32_t entry) {
     shift_out(entry);
-    valid = dot_bytes(entry, (int)0xFF000000u, valid);
+    valid = dot_bytes(entry, 0xFF, valid);
   }
   // Consume `bits` (<= 31) and refill.
   __device__ __forceinline__ void take(uint32_t bits) {
@@ -245,8 +188,7 @@ constexpr unsigned kFullWarp = 0xFFFFFFFFu;
 
 // The rest of a pair whose table entry is not a full pair.  The entry still carries its
 // first symbol and that symbol's length, and take_pair(entry) has already shifted that length
-// out of the cursor (and subtracted the entry's flag byte from the bit counter, which is put
-// right here); `before` is the window the entry was looked up with.  Accounts for the first
+// out of the cursor; `before` is the window the entry was looked up with.  Accounts for the first
 // symbol, looks the second one up on its own and consumes it.
 // Returns (e0 | e1 << 8) << 8, the form a full-pair entry has.
 template <typename Reader>
@@ -259,7 +201,6 @@ __device__ __forceinline__ uint32_t finish_slow_pair(Reader& r, uint32_t entry, 
   const uint32_t literal0 = load_shared_u8(t.byte_table + ((before >> (rare_length + 2)) & 255u));
   const uint32_t second = load_shared_u32(entry_address(bits1, t.table));
   const uint32_t literal1 = load_shared_u8(t.byte_table + ((bits1 >> (rare_length + 2)) & 255u));
-  r.valid += (int)(entry >> 24) - (int)(entry & 31u);
   r.refill();
   const uint32_t e0 = (entry & kEscape) ? literal0 : entry_first_symbol(entry);
   const uint32_t e1 = (second & kEscape) ? literal1 : entry_first_symbol(second);
@@ -455,11 +396,6 @@ __device__ __forceinline__ void prepare_block(const OperandShared& sh, const Ope
   __syncthreads();
 }
 
-__device__ __forceinline__ const uint8_t* tail_origin(const OperandView& a) {
-  if (a.mode == 2) return a.tail + a.descriptor[0] + 2 * (int64_t)(*a.count);
-  return a.tail + a.base;
-}
-
 // Per-lane state of a decoding thread, set up after prepare_block.
 struct LaneState {
   LaneReader reader;
@@ -535,63 +471,6 @@ __device__ __forceinline__ void join_row(const uint4& tile_words, uint2 side_lan
   }
 }
 
-struct OpSpec {
-  const float* alpha;
-  const float* beta;
-  int op;
-  int alpha_is_one;
-  int beta_is_one;
-};
-
-__device__ __forceinline__ float bf16_low(uint32_t w) { return __uint_as_float(w << 16); }
-__device__ __forceinline__ float bf16_high(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
-
-__device__ __forceinline__ uint32_t pack_rn(float low, float high) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(low, high);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-
-// torch.lerp(start, end, weight) in float32, as PyTorch's CUDA kernel evaluates it.
-__device__ __forceinline__ float lerp_f32(float start, float end, float weight) {
-  const float d = __fsub_rn(end, start);
-  return fabsf(weight) < 0.5f ? __fmaf_rn(weight, d, start)
-                              : __fmaf_rn(-d, __fsub_rn(1.0f, weight), end);
-}
-// Two lanes of lerp(start, end, weight), rounded to BF16.
-__device__ __forceinline__ uint32_t lerp_pair(uint32_t start, uint32_t end, float weight) {
-  return pack_rn(lerp_f32(bf16_low(start), bf16_low(end), weight),
-                 lerp_f32(bf16_high(start), bf16_high(end), weight));
-}
-
-// Two lanes of `left (op) right`, rounded once to BF16.
-__device__ __forceinline__ uint32_t apply_op(uint32_t left, uint32_t right, int op, bool alpha_one,
-                                             bool beta_one, float alpha, float beta) {
-  if (op == LCT_OP_ADD) {
-    const __nv_bfloat162 r = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&left),
-                                     *reinterpret_cast<const __nv_bfloat162*>(&right));
-    return *reinterpret_cast<const uint32_t*>(&r);
-  }
-  if (op == LCT_OP_MULTIPLY) {
-    const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&left),
-                                     *reinterpret_cast<const __nv_bfloat162*>(&right));
-    return *reinterpret_cast<const uint32_t*>(&r);
-  }
-  if (op == LCT_OP_LERP) return lerp_pair(left, right, alpha);
-  const float l0 = bf16_low(left), l1 = bf16_high(left);
-  const float r0 = bf16_low(right), r1 = bf16_high(right);
-  if (op == LCT_OP_EMA_SQUARE) {
-    const uint32_t scaled = pack_rn(__fmul_rn(l0, alpha), __fmul_rn(l1, alpha));
-    return pack_rn(__fmaf_rn(beta, __fmul_rn(r0, r0), bf16_low(scaled)),
-                   __fmaf_rn(beta, __fmul_rn(r1, r1), bf16_high(scaled)));
-  }
-  if (alpha_one) {
-    if (beta_one) return pack_rn(__fadd_rn(l0, r0), __fadd_rn(l1, r1));
-    return pack_rn(__fmaf_rn(r0, beta, l0), __fmaf_rn(r1, beta, l1));
-  }
-  if (beta_one) return pack_rn(__fmaf_rn(l0, alpha, r0), __fmaf_rn(l1, alpha, r1));
-  return pack_rn(__fmaf_rn(l0, alpha, __fmul_rn(r0, beta)), __fmaf_rn(l1, alpha, __fmul_rn(r1, beta)));
-}
-
 // Load 8 dense BF16 values of one row (zero beyond the tensor's end).
 __device__ __forceinline__ void load_dense8(const uint16_t* other, int64_t at, int64_t numel,
                                             bool vector_ok, uint32_t w[4]) {
@@ -606,123 +485,6 @@ __device__ __forceinline__ void load_dense8(const uint16_t* other, int64_t at, i
     const uint32_t b = at + 2 * k + 1 < numel ? other[at + 2 * k + 1] : 0u;
     w[k] = a | (b << 16);
   }
-}
-
-// Emit one row of results: dense BF16, or side bytes (storage order) plus
-// exponent bytes (logical order) for the encoder.
-__device__ __forceinline__ void store_row(uint32_t r[4], bool compressed, void* output,
-                                          uint8_t* auxiliary, int64_t at, int64_t numel,
-                                          int64_t storage_at, uint32_t q) {
-  if (!compressed) {
-    uint16_t* out = static_cast<uint16_t*>(output);
-    if (at + 8 <= numel) {
-      __stcs(reinterpret_cast<uint4*>(out + at), make_uint4(r[0], r[1], r[2], r[3]));
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        if (at + i < numel) out[at + i] = (uint16_t)(r[i >> 1] >> (16 * (i & 1)));
-    }
-    return;
-  }
-  if (at + 8 > numel) {  // padding counts as +0.0
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (at + i >= numel) r[i >> 1] &= (i & 1) ? 0x0000FFFFu : 0xFFFF0000u;
-  }
-  const uint32_t l03 = prmt(r[0], r[1], 0x6420), h03 = prmt(r[0], r[1], 0x7531);
-  const uint32_t l47 = prmt(r[2], r[3], 0x6420), h47 = prmt(r[2], r[3], 0x7531);
-  const uint32_t e03 = exponent_bytes(l03, h03), e47 = exponent_bytes(l47, h47);
-  const uint32_t c03 = side_bytes(l03, h03), c47 = side_bytes(l47, h47);
-  const uint2 side_lane_order =
-      make_uint2(prmt(c03, c47, pair_selector_low(q)), prmt(c03, c47, pair_selector_high(q)));
-  *reinterpret_cast<uint2*>(static_cast<uint8_t*>(output) + storage_at) = side_lane_order;
-  if (at + 8 <= numel) {
-    *reinterpret_cast<uint2*>(auxiliary + at) = make_uint2(e03, e47);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      if (at + i < numel) auxiliary[at + i] = (uint8_t)((i < 4 ? e03 : e47) >> (8 * (i & 3)));
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Host-side launch helpers
-// ---------------------------------------------------------------------------
-
-static inline int check_shape(int64_t size, int64_t logical_numel, int block_symbols, int steps,
-                       int fixed_words, int rare_length, Shape* g) {
-  if (steps != 128 && steps != 256) return LCT_E_BAD_GEOMETRY;
-  if (block_symbols != steps * kLanes) return LCT_E_BAD_GEOMETRY;
-  if (fixed_words < 2 || fixed_words > 64) return LCT_E_BAD_GEOMETRY;
-  if (rare_length < 0 || rare_length > 8) return LCT_E_BAD_ARGUMENT;
-  if (size <= 0 || size % block_symbols != 0) return LCT_E_BAD_ARGUMENT;
-  if (logical_numel <= 0 || logical_numel > size) return LCT_E_BAD_ARGUMENT;
-  const int64_t blocks = size / block_symbols;
-  if (blocks > 0x7FFFFFFFLL) return LCT_E_TOO_LARGE;
-  g->size = size;
-  g->logical_numel = logical_numel;
-  g->n_blocks = blocks;
-  g->streams = blocks * kLanes;
-  g->block_symbols = block_symbols;
-  g->steps = steps;
-  g->fixed_words = fixed_words;
-  g->rare_length = rare_length;
-  g->lane_mask = lane_mask_now();
-  return 0;
-}
-
-static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
-
-static inline int view_of(const lct_operand* in, OperandView* v) {
-  if (in == nullptr || in->encoded == nullptr || in->side == nullptr || in->center == nullptr ||
-      in->pair_table == nullptr)
-    return LCT_E_NULL_POINTER;
-  if (!aligned16(in->side) || !aligned16(in->pair_table) || !aligned16(in->encoded))
-    return LCT_E_ALIGNMENT;
-  const lct_overflow& o = in->overflow;
-  if (o.mode < 0 || o.mode > 2) return LCT_E_BAD_ARGUMENT;
-  if (o.mode != 0 && (o.blocks == nullptr || o.tail == nullptr || o.lanes == nullptr ||
-                      o.starts == nullptr))
-    return LCT_E_NULL_POINTER;
-  if (o.mode == 2 && (o.descriptor == nullptr || o.count == nullptr)) return LCT_E_NULL_POINTER;
-  v->encoded = reinterpret_cast<const uint32_t*>(in->encoded);
-  v->side = in->side;
-  v->center = in->center;
-  v->pair_table = in->pair_table;
-  v->lanes = o.lanes;
-  v->starts = o.starts;
-  v->tail = o.tail;
-  v->descriptor = o.descriptor;
-  v->count = o.count;
-  v->blocks = o.blocks;
-  v->base = o.base;
-  v->mode = o.mode;
-  return 0;
-}
-
-// Operation code and its scalars: which of alpha / beta the kernels will read.
-static inline int check_op(int op, const float* alpha, const float* beta, int* alpha_is_one,
-                           int* beta_is_one) {
-  if (op < LCT_OP_ADD || op > LCT_OP_EMA_SQUARE) return LCT_E_BAD_ARGUMENT;
-  if (op == LCT_OP_SCALAR_MUL_ADD) {
-    if (!*alpha_is_one && alpha == nullptr) return LCT_E_NULL_POINTER;
-    if (!*beta_is_one && beta == nullptr) return LCT_E_NULL_POINTER;
-  } else if (op == LCT_OP_LERP) {
-    if (alpha == nullptr) return LCT_E_NULL_POINTER;
-    *alpha_is_one = 0;
-    *beta_is_one = beta == nullptr;  // beta: weight of the Nesterov direction, when one is emitted
-  } else if (op == LCT_OP_EMA_SQUARE) {
-    if (alpha == nullptr || beta == nullptr) return LCT_E_NULL_POINTER;
-    *alpha_is_one = *beta_is_one = 0;
-  } else {
-    *alpha_is_one = *beta_is_one = 1;
-  }
-  return 0;
-}
-
-template <typename Kernel>
-static inline int opt_in_shared(Kernel kernel, size_t bytes) {
-  return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 }  // namespace lct

@@ -59,7 +59,7 @@ struct BlockEncoder {
   int64_t block;
   uint32_t table;
   int wide_rows;  // rows, in whole chunks, that may be read as two-value words
-  LaneWriter a, b;
+  LaneWriter lanes[2];
 
   // What the two lanes append for one row pair, and its side bytes.
   struct Pair {
@@ -85,11 +85,11 @@ struct BlockEncoder {
   template <bool kChecked>
   __device__ __forceinline__ void append(const Pair& p, int step, uint32_t budget_bits) {
     if (kChecked) {
-      a.append_checked(p.a0, p.a1, step, budget_bits);
-      b.append_checked(p.b0, p.b1, step, budget_bits);
+      lanes[0].append_checked(p.a0, p.a1, step, budget_bits);
+      lanes[1].append_checked(p.b0, p.b1, step, budget_bits);
     } else {
-      a.append(p.a0, p.a1);
-      b.append(p.b0, p.b1);
+      lanes[0].append(p.a0, p.a1);
+      lanes[1].append(p.b0, p.b1);
     }
   }
   // The words of the chunk at step0, all requested together: loads requested one by one between
@@ -152,7 +152,7 @@ struct BlockEncoder {
       request(even, 0);
       request(odd, kChunkRows);
       Pair now = look_up(even[0], even[1]);
-      auto near = [&] { return __any_sync(0xFFFFFFFFu, max(a.bits(), b.bits()) + kChunkBits > budget_bits); };
+      auto near = [&] { return __any_sync(0xFFFFFFFFu, max(lanes[0].bits(), lanes[1].bits()) + kChunkBits > budget_bits); };
 #pragma unroll 1
       for (int step0 = 0; step0 < wide_rows; step0 += 2 * kChunkRows) {
         if (prefetches && step0 + kPrefetchRows + kPrefetchPortion <= wide_rows)
@@ -219,13 +219,13 @@ __device__ __forceinline__ void encode_block(const void* __restrict__ src, bool 
   BlockEncoder<kPrecomputed, kLaneMask> encoder{
       static_cast<const char*>(src) + block_base * (kPrecomputed ? 1 : 2),
       side + block_base + 2 * tid, g, block, 0u,
-      src_word_ok ? full_rows / kChunkRows * kChunkRows : 0, {}, {}};
+      src_word_ok ? full_rows / kChunkRows * kChunkRows : 0, {}};
   // A full block of an aligned source is fetched ahead; the first portions now, with everything
   // up to the table still to come.
   const bool prefetches = !kPrecomputed && tid == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
   if (prefetches && encoder.wide_rows >= kPrefetchRows)
     prefetch_l2(encoder.rows, kPrefetchRows * kRowBytes);
-  clear_image(image, g.fixed_words);
+  clear_image<kPairThreads>(image, g.fixed_words);
   if (block == 0 && tid < 4) encoded[g.streams * g.fixed_words + tid] = 0u;  // trailing pad words
   if (!kPrecomputed && rows_used < g.steps) {
     uint4* rest = reinterpret_cast<uint4*>(side + block_base + (int64_t)rows_used * kLanes);
@@ -236,14 +236,14 @@ __device__ __forceinline__ void encode_block(const void* __restrict__ src, bool 
   // kernel that is still running when this grid was launched with programmatic stream
   // serialisation (lct_compress): wait for it only now.
   cudaGridDependencySynchronize();
-  load_encode_table(sh.table, shifted_encode);
+  load_encode_table<kPairThreads>(sh.table, shifted_encode);
   __syncthreads();
 
-  encoder.a.open(shared_address(image + 2 * tid));
-  encoder.b.open(shared_address(image + 2 * tid + 1));
+  encoder.lanes[0].open(shared_address(image + 2 * tid));
+  encoder.lanes[1].open(shared_address(image + 2 * tid + 1));
   encoder.table = after_barrier(shared_address(sh.table));
   encoder.run(rows_used, prefetches);
-  finish_block(encoder.a, encoder.b, image, sh.scan, encoded, extra_starts, summaries, block,
+  finish_block<kPairThreads>(encoder.lanes, image, sh.scan, encoded, extra_starts, summaries, block,
                g.n_blocks, g.streams, g.steps, g.fixed_words);
 }
 

@@ -92,49 +92,57 @@ static_assert(kLanes * 4 == 1024, "LaneWriter steps from image row to image row"
 // More bits than a chunk can add: lanes further than this from their budget need no check.
 constexpr uint32_t kChunkBits = kChunkRows * 16;
 
-// Fill the encode table from the tensor's shifted table (128 threads, no barrier).
+// Fill the encode table from the tensor's shifted table (no barrier).
+template <int kCtaThreads>
 __device__ __forceinline__ void load_encode_table(uint32_t* table, const int32_t* shifted) {
-  table[threadIdx.x] = encode_entry(load_dependent_u32(shifted + threadIdx.x));
-  table[threadIdx.x + kPairThreads] = encode_entry(load_dependent_u32(shifted + threadIdx.x + kPairThreads));
+#pragma unroll
+  for (int i = threadIdx.x; i < 256; i += kCtaThreads)
+    table[i] = encode_entry(load_dependent_u32(shifted + i));
 }
 
-// Clear the payload image of a block (128 threads).
+// Clear the payload image of a block.
+template <int kCtaThreads>
 __device__ __forceinline__ void clear_image(uint32_t* image, int fixed_words) {
   uint4* rows = reinterpret_cast<uint4*>(image);
-  for (int i = threadIdx.x; i < fixed_words * (kLanes / 4); i += kPairThreads)
+  for (int i = threadIdx.x; i < fixed_words * (kLanes / 4); i += kCtaThreads)
     rows[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 // Everything after the last pair of a block: last words, overflow starts, the block's summary,
 // the payload image to global memory (word w of the block's 256 streams is one 1 KB row).
-// `scan`: 2 * kPairWarps shared ints.
-__device__ __forceinline__ void finish_block(LaneWriter& a, LaneWriter& b, const uint32_t* image,
-                                             int* scan, uint32_t* __restrict__ encoded,
+// `writers`: this thread's kLanes / kCtaThreads neighbouring lanes.  `scan`: two shared ints per
+// warp.
+template <int kCtaThreads>
+__device__ __forceinline__ void finish_block(LaneWriter* writers, const uint32_t* image, int* scan,
+                                             uint32_t* __restrict__ encoded,
                                              uint8_t* __restrict__ extra_starts,
                                              int32_t* __restrict__ summaries, int64_t block,
                                              int64_t n_blocks, int64_t streams, int steps,
                                              int fixed_words) {
+  constexpr int kOwn = kLanes / kCtaThreads, kCtaWarps = kCtaThreads / 32;
   const int tid = threadIdx.x;
-  a.close();
-  b.close();
-  extra_starts[block * kLanes + 2 * tid] = (uint8_t)a.extra_start;  // none: 255
-  extra_starts[block * kLanes + 2 * tid + 1] = (uint8_t)b.extra_start;
-  int bad = (a.extra_start >= 0 ? 1 : 0) + (b.extra_start >= 0 ? 1 : 0);
-  int bytes = (a.extra_start >= 0 ? steps - a.extra_start : 0) +
-              (b.extra_start >= 0 ? steps - b.extra_start : 0);
+  int bad = 0, bytes = 0;
+#pragma unroll
+  for (int i = 0; i < kOwn; ++i) {
+    LaneWriter& w = writers[i];
+    w.close();
+    extra_starts[block * kLanes + kOwn * tid + i] = (uint8_t)w.extra_start;  // none: 255
+    bad += w.extra_start >= 0 ? 1 : 0;
+    bytes += w.extra_start >= 0 ? steps - w.extra_start : 0;
+  }
   bad = __reduce_add_sync(0xFFFFFFFFu, bad);
   bytes = __reduce_add_sync(0xFFFFFFFFu, bytes);
-  if ((tid & 31) == 0) { scan[tid >> 5] = bad; scan[kPairWarps + (tid >> 5)] = bytes; }
+  if ((tid & 31) == 0) { scan[tid >> 5] = bad; scan[kCtaWarps + (tid >> 5)] = bytes; }
   __syncthreads();  // also publishes every lane's payload words
   if (tid == 0) {
     int total_bad = 0, total_bytes = 0;
 #pragma unroll
-    for (int w = 0; w < kPairWarps; ++w) { total_bad += scan[w]; total_bytes += scan[kPairWarps + w]; }
+    for (int w = 0; w < kCtaWarps; ++w) { total_bad += scan[w]; total_bytes += scan[kCtaWarps + w]; }
     summaries[block] = total_bad;
     summaries[n_blocks + block] = total_bytes;
   }
   uint32_t* out = encoded + block * kLanes + (tid & 63) * 4;
-  for (int w = tid >> 6; w < fixed_words; w += 2) {
+  for (int w = tid >> 6; w < fixed_words; w += kCtaThreads / 64) {
     const uint4 v = *reinterpret_cast<const uint4*>(&image[w * kLanes + (tid & 63) * 4]);
     __stcs(reinterpret_cast<uint4*>(out + (int64_t)w * streams),
            make_uint4(__brev(v.x), __brev(v.y), __brev(v.z), __brev(v.w)));

@@ -1,6 +1,6 @@
-// Division of a codec block among threads, shared by all kernels that walk bit streams.
+// Division of a codec block among threads.
 //
-// One CTA of 128 threads per block; thread t owns the two neighbouring lanes 2t and 2t + 1.
+// The encoder: one CTA of 128 threads per block; thread t owns the two neighbouring lanes 2t and 2t + 1.
 // The lane mapping XORs a lane with an even mask, and rows 2k and 2k + 1 share their mask, so in
 // every row a thread's two lanes are two neighbouring columns (in order), and a warp's 64 lanes
 // are one aligned group of 64 columns.  A thread therefore handles whole 32-bit words of the
@@ -40,6 +40,25 @@ template <int kLaneMask>
 __device__ __forceinline__ uint32_t chunk_word(uint32_t offset, int k, int lane_mask) {
   const int mask = kLaneMask >= 0 ? kLaneMask : lane_mask;
   return offset ^ (uint32_t)(((2 * k) & mask) * 2);
+}
+
+// The other split, of the kernels that read bit streams: one CTA of 256 threads per block, one
+// lane per thread (twice the warps to hide the walk's latency).  Two neighbouring threads' lanes
+// are two neighbouring columns in every row, so the two exchange exponents with one shuffle per
+// row pair, after which the even thread has both columns of the pair's first row and the odd one
+// those of its second: whole 32-bit words of the dense tensor again, 64-byte segments per warp.
+
+// Element offset inside the block of this thread's word in the chunk that starts at `step0`: the
+// columns of its lane and its neighbour's, in the even or odd rows; see word_at.
+__device__ __forceinline__ uint32_t word_offset(int64_t row0, int step0, int lane_mask) {
+  const uint32_t moved = (threadIdx.x & 254u) ^ (uint32_t)((row0 + step0) & lane_mask);
+  return (step0 + (threadIdx.x & 1u)) * kLanes + moved;
+}
+// ... in row pair k of that chunk.
+template <int kLaneMask>
+__device__ __forceinline__ uint32_t word_at(uint32_t offset, int k, int lane_mask) {
+  const int mask = kLaneMask >= 0 ? kLaneMask : lane_mask;
+  return (offset ^ (uint32_t)((2 * k) & mask)) + (uint32_t)(2 * k * kLanes);
 }
 
 // ---- shared memory by 32-bit address --------------------------------------
@@ -84,10 +103,10 @@ __device__ __forceinline__ void prefetch_l2(const void* address, uint32_t bytes)
 
 // a + sum over the four bytes of e (unsigned) * w (signed): with w = -1 in one byte this
 // subtracts that byte of e from a.
-__device__ __forceinline__ uint32_t dot_bytes(uint32_t e, int w, uint32_t a) {
+__device__ __forceinline__ int dot_bytes(uint32_t e, int w, int a) {
   int d;
-  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(e), "r"(w), "r"((int)a));
-  return (uint32_t)d;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(e), "r"(w), "r"(a));
+  return d;
 }
 
 // a where the mask is set, else b: one three-input logic operation.

@@ -153,8 +153,7 @@ __device__ __forceinline__ void update_sample_chunk(const OperandView& a, const 
   // Same jittered position as the center estimate (one per equal slice of the tensor).
   const int64_t pos = sample_position(idx, n);
   const uint32_t right = other[pos];
-  const float alpha = spec.alpha_is_one ? 1.0f : *spec.alpha;
-  const float beta = spec.beta_is_one ? 1.0f : *spec.beta;
+  const Operation operation(spec);
   uint32_t left;
   if (known != nullptr) {
     // A's values at the sample positions were kept when A was made: no stream to walk.
@@ -179,8 +178,7 @@ __device__ __forceinline__ void update_sample_chunk(const OperandView& a, const 
     const uint32_t exponent = tail >= 0 ? (uint32_t)tail : walk_to(table, g, column, step, center);
     left = (exponent << 7) | (side & 0x7Fu) | ((side & 0x80u) << 8);
   }
-  const uint32_t result = apply_op(left, right, spec.op, spec.alpha_is_one != 0,
-                                   spec.beta_is_one != 0, alpha, beta);
+  const uint32_t result = operation(left, right);
   samples[idx] = (uint8_t)((result >> 7) & 0xFFu);
   if (values != nullptr) values[idx] = (uint16_t)result;
 }
@@ -206,8 +204,7 @@ update_center_known_kernel(const uint16_t* __restrict__ other, int64_t n, OpSpec
                            int32_t* shifted_encode, int32_t* shifted_decode) {
   cudaTriggerProgrammaticLaunchCompletion();  // the fused kernel may start its prologue
   const int64_t count = n < kSampleCount ? n : kSampleCount;
-  const float alpha = spec.alpha_is_one ? 1.0f : *spec.alpha;
-  const float beta = spec.beta_is_one ? 1.0f : *spec.beta;
+  const Operation operation(spec);
   int raw[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
@@ -215,8 +212,7 @@ update_center_known_kernel(const uint16_t* __restrict__ other, int64_t n, OpSpec
     raw[k] = -1;
     if (idx < count) {
       const uint32_t right = other[sample_position(idx, n)];
-      const uint32_t result = apply_op(known[idx], right, spec.op, spec.alpha_is_one != 0,
-                                       spec.beta_is_one != 0, alpha, beta) & 0xFFFFu;
+      const uint32_t result = operation(known[idx], right) & 0xFFFFu;
       raw[k] = (int)((result >> 7) & 0xFFu);
       if (values != nullptr) values[idx] = (uint16_t)result;
     }
@@ -311,8 +307,7 @@ __device__ __forceinline__ void update_fused_block(
     encode_table[tid] = make_uint2(packed & 0xFFFFFu, packed >> 20);
   });  // ends with a block barrier
 
-  const float alpha = spec.alpha_is_one ? 1.0f : *spec.alpha;
-  const float beta = spec.beta_is_one ? 1.0f : *spec.beta;
+  const Operation operation(spec);
   // A job table comes from the caller's device memory: an unaligned by-product pointer takes
   // the scalar stores, a missing one is skipped.
   const bool dense_vector_ok = (reinterpret_cast<uintptr_t>(dense_out) & 15u) == 0;
@@ -367,8 +362,7 @@ __device__ __forceinline__ void update_fused_block(
         join_row(words, side_in[u][half], selectors, half == 1, left);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          result[k] = apply_op(left[k], right[k], spec.op, spec.alpha_is_one != 0,
-                               spec.beta_is_one != 0, alpha, beta);
+          result[k] = operation(left[k], right[k]);
         if (!full_block && l_at + 8 > g.logical_numel) {  // padding counts as +0.0
 #pragma unroll
           for (int i = 0; i < 8; ++i)
@@ -378,7 +372,7 @@ __device__ __forceinline__ void update_fused_block(
           uint32_t dense[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            dense[k] = kEmit == LCT_EMIT_NESTEROV ? lerp_pair(right[k], result[k], beta) : result[k];
+            dense[k] = kEmit == LCT_EMIT_NESTEROV ? lerp_pair(right[k], result[k], operation.beta) : result[k];
           if (dense_vector_ok && l_at + 8 <= g.logical_numel) {
             __stcs(reinterpret_cast<uint4*>(dense_out + l_at),
                    make_uint4(dense[0], dense[1], dense[2], dense[3]));

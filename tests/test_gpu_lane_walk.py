@@ -1,0 +1,51 @@
+"""The walk of the bit streams at the edges of its chunks (16 rows of 256 columns), of a row, of a
+block, and where lanes overflow: bit-exact against the input and the oracle."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+from gpu_helpers import bits_of, to_dev
+from helpers import oracle_compress
+from losslessly_compressed_tensors_b200.comp_format import Distribution, DistType, NoiseLevel
+from losslessly_compressed_tensors_b200.operations import (
+    a_compA_add_B, a_compA_add_compB, compress, decompress, decompress_many,
+)
+from losslessly_compressed_tensors_b200.tensor_buffer import TensorBuffer
+from synth import synth_bf16
+
+pytestmark = pytest.mark.gpu
+
+CHUNK = 16 * 256
+SIZES = [1, 2, 255, 257, 511, CHUNK - 1, CHUNK, CHUNK + 1, 3 * CHUNK + 257, 32768 - 1, 32768 + 1,
+         65536 + 7 * CHUNK + 513]
+CODEBOOKS = {
+    "short": Distribution(DistType.GAUSSIAN),                                    # 128 steps
+    "long": Distribution(DistType.LAPLACE, zero_prob=0.0),                       # 256 steps
+    "loose": Distribution(DistType.GAUSSIAN, noise_level=NoiseLevel.HIGH),       # budget never met
+}
+
+
+@pytest.mark.parametrize("n", SIZES)
+@pytest.mark.parametrize("codebook", sorted(CODEBOOKS))
+@pytest.mark.parametrize("kind", ["normal", "outliers", "wide"])
+def test_walk(oracle, n, codebook, kind):
+    dist = CODEBOOKS[codebook]
+    bits, right, third = synth_bf16(n, 5, kind), synth_bf16(n + 1, 6, "normal", -2), synth_bf16(n, 7, kind)
+    buffer = TensorBuffer(1 << 20)
+    a, b = compress(to_dev(bits), dist, buffer), compress(to_dev(third), dist, buffer)
+    assert np.array_equal(bits_of(decompress(a)), bits)
+    for got, want in zip(decompress_many([b, a]), (third, bits)):
+        assert np.array_equal(bits_of(got), want)
+    want_a = oracle_compress(oracle, bits, dist, oracle.new_arena(1 << 20))
+    alpha = torch.tensor([0.95], dtype=torch.float32, device="cuda")
+    wide = to_dev(right)
+    for offset in (0, 1):  # the dense operand at 16 and at 2 bytes alignment
+        result = a_compA_add_B(a, alpha, wide[offset:offset + n])
+        expect = oracle.pointwise(want_a, right[offset:offset + n], oracle.OP_SCALED, 0.95,
+                                  alpha_is_one=False)
+        assert np.array_equal(bits_of(result).view(np.uint16), expect)
+    dual = a_compA_add_compB(a, alpha, b)
+    expect = oracle.pointwise(want_a, third, oracle.OP_SCALED, 0.95, alpha_is_one=False)
+    assert np.array_equal(bits_of(dual).view(np.uint16), expect)
