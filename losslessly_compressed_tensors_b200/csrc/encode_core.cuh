@@ -19,35 +19,7 @@ __device__ __forceinline__ uint2 load_shared_code(uint32_t table, uint32_t expon
 // construction and, when the pair that moved the position from `pos` to `next` left that word,
 // stores it - as predicated instructions, no branch.
 //
-// ... its column of the block's shared payload image,
-struct SharedWordSink {
-  uint32_t column;  // shared address of word 0 of this lane
-  __device__ __forceinline__ uint32_t address(int pos) const {
-    return column + ((uint32_t)pos & ~31u) * (uint32_t)(kLanes * 4 / 32);
-  }
-  __device__ __forceinline__ void store(int pos, uint32_t word) const {
-    asm volatile("st.shared.u32 [%0], %1;" ::"r"(address(pos)), "r"(word) : "memory");
-  }
-  // lo |= code << (pos & 31); when the pair left the word `pos` is in, store that word and start
-  // the next one with the bits of `code` that did not fit (none when pos is word aligned).
-  __device__ __forceinline__ void append(int pos, int next, uint32_t code, uint32_t& lo) const {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b32 t, d, w;\n\t"
-        "shf.l.wrap.b32 t, 0, %1, %2;\n\t"
-        "or.b32 %0, %0, t;\n\t"
-        "xor.b32 d, %2, %3;\n\t"
-        "setp.ge.u32 p, d, 32;\n\t"
-        "and.b32 w, %2, -32;\n\t"
-        "mad.lo.u32 w, w, 32, %4;\n\t"
-        "@p st.shared.u32 [w], %0;\n\t"
-        "@p shf.l.wrap.b32 %0, %1, 0, %2;\n\t"
-        "}"
-        : "+r"(lo)
-        : "r"(code), "r"(pos), "r"(next), "r"(column)
-        : "memory");
-  }
-};
-// ... or straight to the payload in global memory (row stride = number of streams).
+// Straight to the payload in global memory (row stride = number of streams).
 struct GlobalWordSink {
   uint32_t* column;
   int64_t stride;

@@ -307,7 +307,8 @@ __device__ __forceinline__ void update_fused_block(
     encode_table[tid] = make_uint2(packed & 0xFFFFFu, packed >> 20);
   });  // ends with a block barrier
 
-  const Operation operation(spec);
+  const float alpha = spec.alpha_is_one ? 1.0f : *spec.alpha;
+  const float beta = spec.beta_is_one ? 1.0f : *spec.beta;
   // A job table comes from the caller's device memory: an unaligned by-product pointer takes
   // the scalar stores, a missing one is skipped.
   const bool dense_vector_ok = (reinterpret_cast<uintptr_t>(dense_out) & 15u) == 0;
@@ -362,7 +363,8 @@ __device__ __forceinline__ void update_fused_block(
         join_row(words, side_in[u][half], selectors, half == 1, left);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          result[k] = operation(left[k], right[k]);
+          result[k] = apply_op(left[k], right[k], spec.op, spec.alpha_is_one != 0,
+                               spec.beta_is_one != 0, alpha, beta);
         if (!full_block && l_at + 8 > g.logical_numel) {  // padding counts as +0.0
 #pragma unroll
           for (int i = 0; i < 8; ++i)
@@ -372,7 +374,7 @@ __device__ __forceinline__ void update_fused_block(
           uint32_t dense[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            dense[k] = kEmit == LCT_EMIT_NESTEROV ? lerp_pair(right[k], result[k], operation.beta) : result[k];
+            dense[k] = kEmit == LCT_EMIT_NESTEROV ? lerp_pair(right[k], result[k], beta) : result[k];
           if (dense_vector_ok && l_at + 8 <= g.logical_numel) {
             __stcs(reinterpret_cast<uint4*>(dense_out + l_at),
                    make_uint4(dense[0], dense[1], dense[2], dense[3]));
