@@ -77,7 +77,7 @@ __device__ __forceinline__ void decode_block(const OperandView& a, const Shape& 
   const ReaderShared sh = carve_reader(smem_raw, 0, 1, g.fixed_words, kRingBytes);
   // Rows of pure padding (the tail of a ragged or tiny tensor) have nothing to decode or store.
   const int rows_used = rows_in_use(g, block);
-  BlockDecoder<kLaneMask> decoder{g, block * g.steps, {out + block_base, g.logical_numel - block_base},
+  BlockDecoder<kLaneMask> decoder{g, block * g.steps, {out + block_base, elements_left(g, block)},
                                   {}, {}, {}};
   decoder.sides.open(smem_raw + kTableBytes, a.side + block_base, rows_used);
   stage_operand(sh, a, g, block);
@@ -216,8 +216,8 @@ struct BlockPointwise {
       return;
     }
     if (guarded) {
-      if ((int64_t)at >= out.left) result = 0u;
-      else if ((int64_t)at + 1 >= out.left) result &= 0xFFFFu;
+      if ((int)at >= out.left) result = 0u;
+      else if ((int)at + 1 >= out.left) result &= 0xFFFFu;
     }
     uint32_t sides, exponents;
     split_words(result, 0u, &sides, &exponents);
@@ -284,12 +284,12 @@ pointwise_kernel(OperandView a, OperandView b, Shape g_in, const uint16_t* other
   const int64_t block = blockIdx.x;
   const int tid = threadIdx.x;
   const int64_t block_base = block * (int64_t)g.block_symbols;
-  const int64_t left = g.logical_numel - block_base;
+  const int left = elements_left(g, block);
   const int rows_used = rows_in_use(g, block);
   uint8_t* side_out = static_cast<uint8_t*>(output) + block_base;
   BlockPointwise<kDual, kLaneMask> work{
       g, Operation(spec), block * g.steps, {other + (kDual ? 0 : block_base), left},
-      other_word_ok ? (int)min((int64_t)g.steps, left / kLanes) / kWalkRows * kWalkRows : 0, compressed,
+      other_word_ok ? min(g.steps, left / kLanes) / kWalkRows * kWalkRows : 0, compressed,
       {static_cast<uint16_t*>(output) + (compressed ? 0 : block_base), left},
       side_out + own_bytes(), {auxiliary + (compressed ? block_base : 0), left}, rows_used, {}, {}, {},
       {}, {}};

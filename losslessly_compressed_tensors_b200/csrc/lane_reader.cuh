@@ -11,7 +11,6 @@ namespace lct {
 // Rows per unrolled chunk of a walk.
 constexpr int kWalkPairs = 8;
 constexpr int kWalkRows = 2 * kWalkPairs;
-constexpr uint32_t kWalkBits = kWalkRows * 16;  // more bits than a chunk of a result can add
 
 // Shared memory of a reading CTA with n operands (n = 2 only for the fused operation on two
 // compressed tensors):
@@ -28,12 +27,13 @@ constexpr uint32_t kWalkBits = kWalkRows * 16;  // more bits than a chunk of a r
 // them is harmless; a lane's fetch address is pulled back to a row next to the image once per
 // kClampPairs pairs and cannot leave the CTA's memory in between, whatever the stream holds.
 struct __align__(16) ReaderHead {
-  int32_t overflow_offset[kLanes];
+  uint16_t overflow_offset[kLanes];  // from the block's first tail byte: below steps * kLanes
   uint16_t overflow_start[kLanes];
   uint8_t index_to_byte[256];
+  const uint8_t* tail;               // the block's first tail byte
   int scan[36];
 };
-constexpr size_t kReaderHeadBytes = 2048;
+constexpr size_t kReaderHeadBytes = 1536;
 static_assert(sizeof(ReaderHead) <= kReaderHeadBytes, "head must fit its slot");
 
 constexpr uint32_t kWordRow = kLanes * 4;  // bytes of one word row of the image
@@ -100,6 +100,7 @@ __device__ __forceinline__ void stage_operand(const ReaderShared& sh, const Oper
   head.index_to_byte[tid] = (uint8_t)index_to_exponent_byte((uint32_t)tid, center);
   head.overflow_start[tid] = (uint16_t)g.steps;
   if (count <= 0) return;  // uniform across the CTA
+  if (tid == 0) head.tail = tail_origin(a) + byte_base;
   int lane = 0, length = 0;
   if (tid < count) {
     lane = a.lanes[lane_at + tid];
@@ -110,7 +111,7 @@ __device__ __forceinline__ void stage_operand(const ReaderShared& sh, const Oper
   const int prefix = block_exclusive_scan(length, head.scan, &unused);
   if (tid < count) {
     head.overflow_start[lane] = (uint16_t)(g.steps - length);
-    head.overflow_offset[lane] = byte_base + prefix;
+    head.overflow_offset[lane] = (uint16_t)prefix;
   }
 }
 
@@ -177,9 +178,8 @@ __device__ __forceinline__ uint32_t look_up_entry(uint32_t table, uint32_t windo
 // 1 and 2, whatever else is in it.
 struct LaneWalk {
   LaneCursor cursor;
-  int coded;            // leading steps of this lane that are in the bit stream
-  int tail_from;        // steps from here on come from the raw tail
-  const uint8_t* tail;
+  int coded;  // leading steps of this lane that are in the bit stream
+  const ReaderHead* head;
   uint32_t table;       // shared address of the two-symbol table
   uint32_t byte_table;  // shared address of index_to_byte[256]
   int rare_shift;       // where an escape's literal is in the window it was looked up with
@@ -192,15 +192,13 @@ struct LaneWalk {
     byte_table = shared_address(sh.head->index_to_byte);
     rare_shift = g.rare_length + 2;
     cursor.open(sh.image, lane, g.fixed_words);
-    tail_from = sh.head->overflow_start[lane];
-    coded = min(tail_from, valid_steps_of(block, lane, g.steps, g.block_symbols, g.logical_numel,
-                                          g.lane_mask));
-    tail = nullptr;
-    if (tail_from < g.steps) tail = tail_origin(view) + sh.head->overflow_offset[lane];
+    head = sh.head;
+    coded = min((int)head->overflow_start[lane],
+                valid_steps_of(block, lane, g.steps, g.block_symbols, g.logical_numel, g.lane_mask));
   }
   // All rows of the chunk at step0 are in the streams of all lanes of the warp.
-  __device__ __forceinline__ bool whole_chunk(int step0) const {
-    return __all_sync(0xFFFFFFFFu, step0 + kWalkRows <= coded);
+  __device__ __forceinline__ bool whole_chunk(int step0, int rows = kWalkRows) const {
+    return __all_sync(0xFFFFFFFFu, step0 + rows <= coded);
   }
   __device__ __forceinline__ uint32_t literal(uint32_t window) const {
     return load_shared_u8(byte_table + ((window >> rare_shift) & 255u));
@@ -234,10 +232,12 @@ struct LaneWalk {
     if (k & 1) cursor.refill();  // two full pairs take at most 24 bits: one refill serves both
     return entry;
   }
-  // Tail bytes of the pair at `step`, if it is in the tail (before the offset of 127).
+  // Tail bytes of the pair at `step`, if it is in the tail (before the offset of 127).  Where the
+  // tail starts is read again each time: rarely needed, it would hold registers throughout.
   __device__ __forceinline__ uint32_t tail_pair(int step, int steps) const {
-    if (step < tail_from || step >= steps) return 0u;
-    const uint8_t* t = tail + (step - tail_from);
+    const int from = head->overflow_start[threadIdx.x];
+    if (step < from || step >= steps) return 0u;
+    const uint8_t* t = head->tail + (head->overflow_offset[threadIdx.x] + step - from);
     return (uint32_t)t[0] | ((uint32_t)t[1] << 16);
   }
   // The pair at `step`, wherever its symbols are; `raw`: tail_pair() of that step.
@@ -255,16 +255,16 @@ struct LaneWalk {
       cursor.refill();
       return entry;
     }
-    if (step < tail_from) return 0u;
+    if (step < head->overflow_start[threadIdx.x]) return 0u;
     return prmt(raw + 0x007F007Fu, 0u, 0x4204);  // bytes 0 and 2 to bytes 1 and 2
   }
   // The pairs of a chunk in which some lane's stream ends, or has ended.  `emit(k, entry)` gets
   // them one after the other; tail bytes are requested a pair ahead.
   template <typename Emit>
-  __device__ __forceinline__ void read_chunk(int step0, int steps, Emit emit) {
+  __device__ __forceinline__ void read_chunk(int step0, int steps, Emit emit, int pairs = kWalkPairs) {
     uint32_t ahead = tail_pair(step0, steps);
 #pragma unroll 1
-    for (int k = 0; k < kWalkPairs; ++k) {
+    for (int k = 0; k < pairs; ++k) {
       const uint32_t raw = ahead;
       ahead = tail_pair(step0 + 2 * k + 2, steps);
       emit(k, read_any(step0 + 2 * k, raw));
@@ -287,38 +287,43 @@ struct RowExchange {
   }
 };
 
+constexpr int kMaxLeft = 1 << 20;  // more than a block has
+__device__ __forceinline__ int elements_left(const Shape& g, int64_t block) {
+  return (int)min((int64_t)kMaxLeft, g.logical_numel - block * (int64_t)g.block_symbols);
+}
+
 // Where a thread's words of a dense tensor are: rows of the block from `rows` on, a word of two
 // neighbouring columns per row.  Offsets are in elements.
 template <typename Element>
 struct DenseWords {
   Element* rows;
-  int64_t left;  // elements from `rows` to the tensor's end
+  int left;  // elements from `rows` to the tensor's end, at most kMaxLeft
 
   __device__ __forceinline__ void store(uint32_t at, uint32_t word) const {
     __stcs(reinterpret_cast<uint32_t*>(rows + at), word);
   }
   __device__ __forceinline__ void store_guarded(uint32_t at, uint32_t word) const {
-    if ((int64_t)at < left) rows[at] = (uint16_t)word;
-    if ((int64_t)at + 1 < left) rows[at + 1] = (uint16_t)(word >> 16);
+    if ((int)at < left) rows[at] = (uint16_t)word;
+    if ((int)at + 1 < left) rows[at + 1] = (uint16_t)(word >> 16);
   }
   __device__ __forceinline__ uint32_t load(uint32_t at) const { return load_ahead_u32(rows + at); }
   __device__ __forceinline__ uint32_t load_guarded(uint32_t at) const {
-    const uint32_t low = (int64_t)at < left ? rows[at] : 0u;
-    const uint32_t high = (int64_t)at + 1 < left ? rows[at + 1] : 0u;
+    const uint32_t low = (int)at < left ? rows[at] : 0u;
+    const uint32_t high = (int)at + 1 < left ? rows[at + 1] : 0u;
     return low | (high << 16);
   }
 };
 
 // Move the word of the pair that was just finished out of a chunk's buffer.
-__device__ __forceinline__ void next_pair(uint32_t (&words)[kWalkPairs]) {
+template <int kPairs>
+__device__ __forceinline__ void next_pair(uint32_t (&words)[kPairs]) {
 #pragma unroll
-  for (int k = 0; k + 1 < kWalkPairs; ++k) words[k] = words[k + 1];
+  for (int k = 0; k + 1 < kPairs; ++k) words[k] = words[k + 1];
 }
 
 // Rows of a block that hold elements, in whole chunks.
 __device__ __forceinline__ int rows_in_use(const Shape& g, int64_t block) {
-  const int64_t left = g.logical_numel - block * (int64_t)g.block_symbols;
-  const int in_block = (int)max((int64_t)0, min((int64_t)g.block_symbols, left));
+  const int in_block = max(0, min(g.block_symbols, elements_left(g, block)));
   return (in_block + kWalkRows * kLanes - 1) / (kWalkRows * kLanes) * kWalkRows;
 }
 

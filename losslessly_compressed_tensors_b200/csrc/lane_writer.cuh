@@ -89,6 +89,63 @@ struct LaneWriter {
 };
 static_assert(kLanes * 4 == 1024, "LaneWriter steps from image row to image row");
 
+// The same with finished words going straight to the payload in global memory, for kernels whose
+// shared memory an image would cost resident CTAs (a warp's lanes write neighbouring words of the
+// same payload rows; L2 merges them).
+struct GlobalLaneWriter {
+  uint32_t low, high;  // the last 64 bits of the stream
+  uint32_t pos;        // bits so far in the low 16 bits
+  uint32_t* at;        // next payload word of this lane
+  int64_t row_bytes;   // from one payload word of a lane to the next
+  int extra_start;     // first overflowing step, -1 = none
+
+  __device__ __forceinline__ void open(uint32_t* column, int64_t streams) {
+    low = high = pos = 0u;
+    at = column;
+    row_bytes = streams * 4;
+    extra_start = -1;
+  }
+  __device__ __forceinline__ uint32_t bits() const { return pos & 0xFFFFu; }
+  __device__ __forceinline__ void append(uint32_t first, uint32_t second) {
+    high = __funnelshift_l(low, high, first);
+    low = __funnelshift_l(first, low, first);
+    high = __funnelshift_l(low, high, second);
+    low = __funnelshift_l(second, low, second);
+    const uint32_t next = pos + first + second;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b32 d, w;\n\t"
+        "lop3.b32 d, %1, %2, 32, 0x28;\n\t"  // (pos ^ next) & 32
+        "setp.ne.u32 p, d, 0;\n\t"
+        "@p shf.r.wrap.b32 w, %3, %4, %2;\n\t"
+        "@p brev.b32 w, w;\n\t"
+        "@p st.global.u32 [%0], w;\n\t"
+        "@p add.s64 %0, %0, %5;\n\t"
+        "}"
+        : "+l"(at)
+        : "r"(pos), "r"(next), "r"(low), "r"(high), "l"(row_bytes)
+        : "memory");
+    pos = next;
+  }
+  __device__ __forceinline__ void append_checked(uint32_t first, uint32_t second, int step,
+                                                 uint32_t budget_bits) {
+    const bool fits = ((pos + first + second) & 0xFFFFu) <= budget_bits;
+    const bool open = extra_start < 0;
+    append(open && fits ? first : 0u, open && fits ? second : 0u);
+    if (open && !fits) extra_start = step;
+  }
+  // The word under construction after the last pair, and zeros up to the budget.
+  __device__ __forceinline__ void close(int fixed_words) {
+    int word = bits() >> 5;
+    char* to = reinterpret_cast<char*>(at);
+    if (pos & 31u) {
+      *reinterpret_cast<uint32_t*>(to) = __brev(low << (32u - (pos & 31u)));
+      to += row_bytes;
+      ++word;
+    }
+    for (; word < fixed_words; ++word, to += row_bytes) *reinterpret_cast<uint32_t*>(to) = 0u;
+  }
+};
+
 // More bits than a chunk can add: lanes further than this from their budget need no check.
 constexpr uint32_t kChunkBits = kChunkRows * 16;
 
@@ -108,32 +165,27 @@ __device__ __forceinline__ void clear_image(uint32_t* image, int fixed_words) {
     rows[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
-// Everything after the last pair of a block: last words, overflow starts, the block's summary,
-// the payload image to global memory (word w of the block's 256 streams is one 1 KB row).
-// `writers`: this thread's kLanes / kCtaThreads neighbouring lanes.  `scan`: two shared ints per
-// warp.
-template <int kCtaThreads>
-__device__ __forceinline__ void finish_block(LaneWriter* writers, const uint32_t* image, int* scan,
-                                             uint32_t* __restrict__ encoded,
-                                             uint8_t* __restrict__ extra_starts,
-                                             int32_t* __restrict__ summaries, int64_t block,
-                                             int64_t n_blocks, int64_t streams, int steps,
-                                             int fixed_words) {
+// Overflow starts of this thread's neighbouring lanes and the block's summary, with a block barrier
+// between.  `writers`: kLanes / kCtaThreads of them.  `scan`: two shared ints per warp.
+template <int kCtaThreads, typename Writer>
+__device__ __forceinline__ void summarise_block(const Writer* writers, int* scan,
+                                                uint8_t* __restrict__ extra_starts,
+                                                int32_t* __restrict__ summaries, int64_t block,
+                                                int64_t n_blocks, int steps) {
   constexpr int kOwn = kLanes / kCtaThreads, kCtaWarps = kCtaThreads / 32;
   const int tid = threadIdx.x;
   int bad = 0, bytes = 0;
 #pragma unroll
   for (int i = 0; i < kOwn; ++i) {
-    LaneWriter& w = writers[i];
-    w.close();
-    extra_starts[block * kLanes + kOwn * tid + i] = (uint8_t)w.extra_start;  // none: 255
-    bad += w.extra_start >= 0 ? 1 : 0;
-    bytes += w.extra_start >= 0 ? steps - w.extra_start : 0;
+    const int start = writers[i].extra_start;
+    extra_starts[block * kLanes + kOwn * tid + i] = (uint8_t)start;  // none: 255
+    bad += start >= 0 ? 1 : 0;
+    bytes += start >= 0 ? steps - start : 0;
   }
   bad = __reduce_add_sync(0xFFFFFFFFu, bad);
   bytes = __reduce_add_sync(0xFFFFFFFFu, bytes);
   if ((tid & 31) == 0) { scan[tid >> 5] = bad; scan[kCtaWarps + (tid >> 5)] = bytes; }
-  __syncthreads();  // also publishes every lane's payload words
+  __syncthreads();
   if (tid == 0) {
     int total_bad = 0, total_bytes = 0;
 #pragma unroll
@@ -141,6 +193,22 @@ __device__ __forceinline__ void finish_block(LaneWriter* writers, const uint32_t
     summaries[block] = total_bad;
     summaries[n_blocks + block] = total_bytes;
   }
+}
+
+// Everything after the last pair of a block: last words, overflow starts, the block's summary,
+// the payload image to global memory (word w of the block's 256 streams is one 1 KB row).
+template <int kCtaThreads>
+__device__ __forceinline__ void finish_block(LaneWriter* writers, const uint32_t* image, int* scan,
+                                             uint32_t* __restrict__ encoded,
+                                             uint8_t* __restrict__ extra_starts,
+                                             int32_t* __restrict__ summaries, int64_t block,
+                                             int64_t n_blocks, int64_t streams, int steps,
+                                             int fixed_words) {
+  const int tid = threadIdx.x;
+#pragma unroll
+  for (int i = 0; i < kLanes / kCtaThreads; ++i) writers[i].close();
+  // (Its barrier also publishes every lane's payload words.)
+  summarise_block<kCtaThreads>(writers, scan, extra_starts, summaries, block, n_blocks, steps);
   uint32_t* out = encoded + block * kLanes + (tid & 63) * 4;
   for (int w = tid >> 6; w < fixed_words; w += kCtaThreads / 64) {
     const uint4 v = *reinterpret_cast<const uint4*>(&image[w * kLanes + (tid & 63) * 4]);

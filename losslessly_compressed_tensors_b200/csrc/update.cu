@@ -27,6 +27,8 @@
 #include "center.cuh"
 #include "decode_core.cuh"
 #include "encode_core.cuh"
+#include "lane_reader.cuh"
+#include "lane_writer.cuh"
 
 namespace lct {
 
@@ -456,12 +458,226 @@ update_fused_kernel(OperandView a, Shape g, const uint16_t* other, bool other_ve
                                        dense_out, blockIdx.x);
 }
 
+// ---- the same without tiles -------------------------------------------------
+//
+// Form of the batched update: a thread walks its lane (lane_reader.cuh) and appends to its own
+// output stream; neighbouring threads exchange exponents by shuffle on the way to their rows and
+// back.  Fewer instructions per pair than the tile form, but more registers, which leaves three
+// CTAs per SM instead of four (at four, spilling, all of the gain is lost).  Lists of tensors
+// fill the device several times over and gain: 12 x 4096 x 4096 444 -> 400 us, the 8 matrices of
+// two 768-wide layers 53.4 -> 49.7.  A single tensor of 400 to 600 blocks is one wave of the tile
+// form and loses (4096 x 4096 51.9 -> 52.7 us, 8192 x 4096 87.8 -> 92.1): it keeps that form.
+
+// Shared memory of a CTA: [decode table | encode table, scan scratch, ring of side bytes | head,
+// input image].
+struct __align__(16) UpdateShared {
+  uint32_t encode_table[256];
+  int scan[16];
+  unsigned char ring[kRingBytes];
+};
+static inline __host__ __device__ size_t update_walk_shared_bytes(int fixed_words) {
+  return reader_shared_bytes(1, fixed_words, sizeof(UpdateShared));
+}
+
+// One thread of a block: its lane's walk and its lane's output stream, and between them its row of
+// every pair (two neighbouring columns, see lanes.cuh): join, operation, split.  Chunks of 8 rows,
+// half a stage of the ring.
+template <int kLaneMask, int kEmit>
+struct BlockUpdate {
+  const Shape& g;
+  Operation operation;
+  int64_t row0;
+  uint8_t* side_out;
+  DenseWords<const uint16_t> other;
+  int wide_rows;  // rows, in whole chunks, of `other` that may be read as words
+  DenseWords<uint16_t> dense;  // kEmit: the dense by-product (may alias `other`)
+  bool dense_word_ok;
+  uint8_t* spill;  // the block's first element
+  int rows_used;
+  uint32_t encode_table;
+  uint32_t lane_selector;  // see to_lane
+  RowExchange rows;
+  SideRing sides;
+  LaneWalk walk;
+  GlobalLaneWriter writer;
+
+  using Buffer = uint32_t[kChunkPairs];  // words of `other`
+  __device__ __forceinline__ void request(Buffer& right, int step0) const {
+    if (step0 >= rows_used) return;
+    const uint32_t offset = word_offset(row0, step0, g.lane_mask);
+#pragma unroll
+    for (int k = 0; k < kChunkPairs; ++k) {
+      const uint32_t at = word_at<kLaneMask>(offset, k, g.lane_mask);
+      right[k] = step0 < wide_rows ? other.load(at) : other.load_guarded(at);
+    }
+  }
+  // This thread's row of the pair at `step`: its two result exponents (bytes 0 and 1).
+  template <bool kGuarded>
+  __device__ __forceinline__ uint32_t row_exponents(int step, uint32_t at, uint32_t exponents_in,
+                                                    uint32_t from_a, uint32_t right) const {
+    uint32_t result = operation(join_word(exponents_in, from_a), right);
+    if (kGuarded) {  // padding counts as +0.0
+      if ((int)at >= other.left) result = 0u;
+      else if ((int)at + 1 >= other.left) result &= 0xFFFFu;
+    }
+    if (kEmit != LCT_EMIT_NONE && dense.rows != nullptr) {
+      const uint32_t word =
+          kEmit == LCT_EMIT_NESTEROV ? lerp_pair(right, result, operation.beta) : result;
+      if (!kGuarded && dense_word_ok) dense.store(at, word);
+      else dense.store_guarded(at, word);
+    }
+    uint32_t sides_of_row, exponents;
+    split_words(result, 0u, &sides_of_row, &exponents);
+    __stcs(reinterpret_cast<uint16_t*>(side_out + step * kLanes), (uint16_t)sides_of_row);
+    return exponents;
+  }
+  // From rows back to lanes: the even thread takes the even column of both rows, the odd one the
+  // odd column; first row in byte 0, second in byte 1.
+  __device__ __forceinline__ uint32_t to_lane(uint32_t own, uint32_t neighbour) const {
+    return prmt(own, neighbour, lane_selector);
+  }
+  // Raw exponents of an overflowed lane's pair, for the tail pass; `at`: this thread's word.
+  template <bool kGuarded>
+  __device__ __forceinline__ void spill_pair(uint32_t at, uint32_t exponents) const {
+    if (writer.extra_start < 0) return;
+    const uint32_t own = at - (threadIdx.x & 1u) * (kLanes - 1);  // this lane's column, first row
+    if (!kGuarded || (int)own < other.left) spill[own] = (uint8_t)exponents;
+    if (!kGuarded || (int)own + kLanes < other.left) spill[own + kLanes] = (uint8_t)(exponents >> 8);
+  }
+
+  // Every lane of the warp reads whole pairs; unless kChecked it is also further than a chunk from
+  // its budget.  Pair k is read while pair k - 1 is at its row side and pair k - 2 is appended.
+  template <bool kChecked>
+  __device__ __forceinline__ void whole_chunk(int step0, int first_pair, const Buffer& right) {
+    const uint32_t offset = word_offset(row0, step0, g.lane_mask);
+    uint32_t entry = 0u, entry_neighbour = 0u, side = 0u, result = 0u, result_neighbour = 0u;
+    auto row_side = [&](int k) {
+      result = row_exponents<false>(step0 + 2 * k, word_at<kLaneMask>(offset, k, g.lane_mask),
+                                    rows.exponents(entry, entry_neighbour), side, right[k]);
+      result_neighbour = rows.neighbours(result);
+    };
+    auto append = [&](int k) {
+      const uint32_t exponents = to_lane(result, result_neighbour);
+      const uint32_t first = encode_entry_of<0>(encode_table, exponents);
+      const uint32_t second = encode_entry_of<1>(encode_table, exponents);
+      if (kChecked) {
+        writer.append_checked(first, second, step0 + 2 * k, (uint32_t)g.fixed_words * 32u);
+        spill_pair<false>(word_at<kLaneMask>(offset, k, g.lane_mask), exponents);
+      } else {
+        writer.append(first, second);
+      }
+    };
+#pragma unroll
+    for (int k = 0; k < kChunkPairs; ++k) {
+      entry = walk.read_pair(k, [&] {
+        if (k > 1) append(k - 2);
+        if (k > 0) row_side(k - 1);
+      });
+      entry_neighbour = rows.neighbours(entry);
+      side = sides.pair(first_pair + k);
+    }
+    append(kChunkPairs - 2);
+    row_side(kChunkPairs - 1);
+    append(kChunkPairs - 1);
+  }
+  // A chunk in which some lane's input stream ends, pair by pair.
+  __device__ __forceinline__ void partial_chunk(int step0, int first_pair, Buffer& right) {
+    const uint32_t offset = word_offset(row0, step0, g.lane_mask);
+    const int valid = valid_steps_of(row0 / g.steps, threadIdx.x, g.steps, g.block_symbols,
+                                     g.logical_numel, g.lane_mask);
+    walk.read_chunk(step0, g.steps, [&](int k, uint32_t entry) {
+      const int step = step0 + 2 * k;
+      const uint32_t at = word_at<kLaneMask>(offset, k, g.lane_mask);
+      const uint32_t result =
+          row_exponents<true>(step, at, rows.exponents(entry, rows.neighbours(entry)),
+                              sides.pair(first_pair + k), right[0]);
+      const uint32_t exponents = to_lane(result, rows.neighbours(result));
+      const uint32_t first = encode_entry_of<0>(encode_table, exponents);
+      const uint32_t second = encode_entry_of<1>(encode_table, exponents);
+      // Padding carries no bits.
+      writer.append_checked(step < valid ? first : 0u, step + 1 < valid ? second : 0u, step,
+                            (uint32_t)g.fixed_words * 32u);
+      spill_pair<true>(at, exponents);
+      next_pair(right);
+    }, kChunkPairs);
+  }
+  __device__ __forceinline__ void run() {
+    Buffer now, next;
+    request(now, 0);
+#pragma unroll 1
+    for (int step0 = 0; step0 < rows_used; step0 += kChunkRows) {
+      const int first_pair = (step0 & (kWalkRows - 1)) >> 1;
+      request(next, step0 + kChunkRows);
+      if (first_pair == 0) sides.wait();
+      const bool far = writer.bits() + kChunkBits <= (uint32_t)g.fixed_words * 32u;
+      if (!walk.whole_chunk(step0, kChunkRows)) partial_chunk(step0, first_pair, now);
+      else if (__all_sync(0xFFFFFFFFu, far)) whole_chunk<false>(step0, first_pair, now);
+      else whole_chunk<true>(step0, first_pair, now);
+      if (first_pair != 0) sides.advance();
+#pragma unroll
+      for (int k = 0; k < kChunkPairs; ++k) now[k] = next[k];
+    }
+  }
+};
+
+// One codec block of a batch; parameters as for update_fused_block.
+template <int kLaneMask, int kEmit>
+__device__ __forceinline__ void update_walk_block(
+    const OperandView& view, const Shape& g_in, const uint16_t* other, const OpSpec& spec,
+    const int32_t* shifted_encode, uint8_t* side_out, uint32_t* encoded_out, uint8_t* extra_starts,
+    int32_t* summaries, uint8_t* spill, uint16_t* dense_out, int64_t block) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Shape g = g_in;
+  if (kLaneMask >= 0) g.lane_mask = kLaneMask;  // compile-time lane mapping, see BlockDecoder
+  const ReaderShared sh = carve_reader(smem_raw, 0, 1, g.fixed_words, sizeof(UpdateShared));
+  UpdateShared& own = *reinterpret_cast<UpdateShared*>(smem_raw + kTableBytes);
+
+  const int tid = threadIdx.x;
+  const int64_t block_base = block * (int64_t)g.block_symbols;
+  const int left = elements_left(g, block);
+  const int rows_used = rows_in_use(g, block);
+  // The input operand does not depend on the result's center: its payload is staged and its
+  // tables are built before this grid waits for the kernel that writes the shifted encode table.
+  SideRing sides;
+  sides.open(own.ring, view.side + block_base, rows_used);
+  stage_operand(sh, view, g, block);
+  if (block == 0 && tid < 4) encoded_out[g.streams * g.fixed_words + tid] = 0u;  // trailing pad words
+  // Rows of pure padding carry no bits; their side bytes are cleared in one sweep.
+  uint4* rest = reinterpret_cast<uint4*>(side_out + block_base + (int64_t)rows_used * kLanes);
+  for (int i = tid; i < (g.steps - rows_used) * (kLanes / 16); i += kThreads)
+    __stcs(rest + i, make_uint4(0u, 0u, 0u, 0u));
+  cudaGridDependencySynchronize();
+  load_encode_table<kThreads>(own.encode_table, shifted_encode);
+  cp_async_wait_all();
+  __syncthreads();
+
+  const bool word_ok = (reinterpret_cast<uintptr_t>(other) & 3u) == 0;
+  // A job table comes from the caller's device memory: an unaligned by-product pointer takes
+  // the scalar stores, a missing one is skipped.
+  BlockUpdate<kLaneMask, kEmit> work{
+      g, Operation(spec), block * g.steps, side_out + block_base + own_bytes(),
+      {other + block_base, left}, word_ok ? min(g.steps, left / kLanes) / kChunkRows * kChunkRows : 0,
+      {dense_out == nullptr ? nullptr : dense_out + block_base, left},
+      (reinterpret_cast<uintptr_t>(dense_out) & 3u) == 0, spill + block_base, rows_used,
+      after_barrier(shared_address(own.encode_table)), (tid & 1) ? 0x4415u : 0x4440u, {}, {}, {}, {}};
+  work.sides = sides;
+  work.rows.open();
+  work.walk.open(sh, view, g, block);
+  work.writer.open(encoded_out + block * kLanes + tid, g.streams);
+  work.run();
+  work.writer.close(g.fixed_words);
+  summarise_block<kThreads>(&work.writer, own.scan, extra_starts, summaries, block, g.n_blocks, g.steps);
+}
+
+// Resident CTAs per SM the batched kernel is compiled for.
+constexpr int kUpdateWalkMinCtas = 3;
+
 // Every block of every job of a batch: CTA b serves the job whose block range contains b.
 template <int kLaneMask, int kEmit>
-__global__ void __launch_bounds__(kThreads, 4)
+__global__ void __launch_bounds__(kThreads, kUpdateWalkMinCtas)
 update_fused_batch_kernel(const lct_update_job* __restrict__ jobs, int n_jobs, Shape common,
                           OpSpec spec, const int32_t* shifted_encode,
-                          uint8_t* __restrict__ extra_starts, int32_t* __restrict__ summaries) {
+                          uint8_t* extra_starts, int32_t* summaries) {
   const int64_t block = blockIdx.x;
   int lo = 0, hi = n_jobs - 1;
   while (lo < hi) {  // last job with first_block <= block
@@ -469,10 +685,9 @@ update_fused_batch_kernel(const lct_update_job* __restrict__ jobs, int n_jobs, S
     if (jobs[mid].first_block <= block) lo = mid; else hi = mid - 1;
   }
   const lct_update_job& job = jobs[lo];
-  const bool vector_ok = (reinterpret_cast<uintptr_t>(job.other) & 15u) == 0;
-  update_fused_block<kLaneMask, kEmit>(
+  update_walk_block<kLaneMask, kEmit>(
       view_of_update(job.a), shape_of_update(job, common), static_cast<const uint16_t*>(job.other),
-      vector_ok, spec, shifted_encode + 256 * (int64_t)lo, job.side_out,
+      spec, shifted_encode + 256 * (int64_t)lo, job.side_out,
       reinterpret_cast<uint32_t*>(job.encoded_out), extra_starts + job.first_block * kLanes,
       summaries + 4 * job.first_block, job.spill, static_cast<uint16_t*>(job.dense_out),
       block - job.first_block);
@@ -694,7 +909,7 @@ int lct_update_batch_emit(const lct_update_job* jobs, int n_jobs, int64_t total_
   if ((rc = lct::launch_center_batch(jobs, n_jobs, encode_table, decode_table, samples,
                                      shifted_encode, st)))
     return rc;
-  const size_t shared = lct::operand_shared_bytes(fixed_words) + 256 * sizeof(uint2);
+  const size_t shared = lct::update_walk_shared_bytes(fixed_words);
   if (emit < LCT_EMIT_NONE || emit > LCT_EMIT_NESTEROV) return LCT_E_BAD_ARGUMENT;
   if (emit == LCT_EMIT_NESTEROV && (op != LCT_OP_LERP || beta == nullptr)) return LCT_E_BAD_ARGUMENT;
   const bool swizzled = g.lane_mask == 254;

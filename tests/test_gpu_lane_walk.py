@@ -8,11 +8,13 @@ import torch
 
 from gpu_helpers import bits_of, to_dev
 from helpers import oracle_compress
+from losslessly_compressed_tensors_b200.LCTensor import LCTTensor
 from losslessly_compressed_tensors_b200.comp_format import Distribution, DistType, NoiseLevel
 from losslessly_compressed_tensors_b200.operations import (
     a_compA_add_B, a_compA_add_compB, compress, decompress, decompress_many,
 )
 from losslessly_compressed_tensors_b200.tensor_buffer import TensorBuffer
+from losslessly_compressed_tensors_b200.update_plan import UpdatePlan
 from synth import synth_bf16
 
 pytestmark = pytest.mark.gpu
@@ -49,3 +51,26 @@ def test_walk(oracle, n, codebook, kind):
     dual = a_compA_add_compB(a, alpha, b)
     expect = oracle.pointwise(want_a, third, oracle.OP_SCALED, 0.95, alpha_is_one=False)
     assert np.array_equal(bits_of(dual).view(np.uint16), expect)
+
+
+@pytest.mark.parametrize("codebook", sorted(CODEBOOKS))
+@pytest.mark.parametrize("kind", ["normal", "outliers", "wide"])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_batched_update_equals_single_updates(codebook, kind, offset):
+    """The batched update walks lanes, the single one works on tiles: same payload, same result."""
+    dist = CODEBOOKS[codebook]
+    alpha = torch.tensor([0.95], dtype=torch.float32, device="cuda")
+    buffer, reference = TensorBuffer(1 << 22), TensorBuffer(1 << 22)
+    bits = [synth_bf16(n, 20 + i, kind) for i, n in enumerate(SIZES)]
+    together = [LCTTensor(to_dev(b), buffer, dist) for b in bits]
+    alone = [LCTTensor(to_dev(b), reference, dist) for b in bits]
+    plan = UpdatePlan(together, alpha)
+    for step in range(3):
+        grads = [to_dev(synth_bf16(n + 1, 40 + 20 * step + i, kind, step - 1))[offset:offset + n]
+                 for i, n in enumerate(SIZES)]
+        plan.step(grads)
+        for a, b, g in zip(together, alone, grads):
+            b.mul_add_(alpha, g)
+            for part in ("data", "sign_mantissa", "center", "fallback_count"):
+                assert torch.equal(getattr(a.x, part), getattr(b.x, part)), (part, g.numel(), step)
+            assert torch.equal(decompress(a.x).view(torch.int16), decompress(b.x).view(torch.int16))
