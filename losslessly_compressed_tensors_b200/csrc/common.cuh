@@ -7,8 +7,9 @@
 // one XOR mask, and the mask is even, so lanes 2p/2p+1 stay adjacent.  The
 // mask's bits 5..7 move a warp's 32 lanes to another aligned group of 32
 // columns and its bits 1..4 permute them inside that group, so in every row
-// one warp's lanes cover exactly one 64-byte segment of the BF16 row.  That
-// makes the pipeline warp-private: a warp (32 lanes of a block) passes its
+// one warp's lanes cover exactly one 64-byte segment of the BF16 row.  How
+// threads divide a block is said in lanes.cuh; the fused update of a single
+// tensor keeps a warp-private tile form: a warp (32 lanes of a block) passes its
 // data through its own shared-memory tile, 32 rows at a time:
 //
 //     tile[pair p][x] = e(row 2p) | e(row 2p+1) << 8  of lane  x ^ (2p & lane_mask & 6)

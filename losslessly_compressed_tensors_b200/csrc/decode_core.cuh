@@ -1,8 +1,6 @@
-// Device building blocks shared by the decoder, the fused pointwise kernels and
-// the fused update kernel: operand views, the per-CTA prologue (staging of the
-// payload and of the center's two-symbol table, overflow map), the lane-side
-// stream cursor and tile decoder, the row-side BF16 join/split, the arithmetic
-// of the fused operations, and the host-side argument checks.
+// Decoder side of the tile form that the fused update of a single tensor keeps: the per-CTA
+// prologue (staging of the payload and of the center's two-symbol table, overflow map), the
+// lane-side stream cursor and tile decoder, and the row-side BF16 join.
 #pragma once
 
 #include "lanes.cuh"
