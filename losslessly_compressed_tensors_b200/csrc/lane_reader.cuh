@@ -288,8 +288,11 @@ struct RowExchange {
 };
 
 constexpr int kMaxLeft = 1 << 20;  // more than a block has
+// Elements from the block's first on, 0 to kMaxLeft.  Bounded on both sides: storage may hold any
+// number of blocks of pure padding, and how far a block lies behind the end need not fit 32 bits.
 __device__ __forceinline__ int elements_left(const Shape& g, int64_t block) {
-  return (int)min((int64_t)kMaxLeft, g.logical_numel - block * (int64_t)g.block_symbols);
+  const int64_t left = g.logical_numel - block * (int64_t)g.block_symbols;
+  return (int)max((int64_t)0, min((int64_t)kMaxLeft, left));
 }
 
 // Where a thread's words of a dense tensor are: rows of the block from `rows` on, a word of two
@@ -297,7 +300,7 @@ __device__ __forceinline__ int elements_left(const Shape& g, int64_t block) {
 template <typename Element>
 struct DenseWords {
   Element* rows;
-  int left;  // elements from `rows` to the tensor's end, at most kMaxLeft
+  int left;  // elements_left()
 
   __device__ __forceinline__ void store(uint32_t at, uint32_t word) const {
     __stcs(reinterpret_cast<uint32_t*>(rows + at), word);
@@ -323,7 +326,7 @@ __device__ __forceinline__ void next_pair(uint32_t (&words)[kPairs]) {
 
 // Rows of a block that hold elements, in whole chunks.
 __device__ __forceinline__ int rows_in_use(const Shape& g, int64_t block) {
-  const int in_block = max(0, min(g.block_symbols, elements_left(g, block)));
+  const int in_block = min(g.block_symbols, elements_left(g, block));
   return (in_block + kWalkRows * kLanes - 1) / (kWalkRows * kLanes) * kWalkRows;
 }
 

@@ -9,7 +9,11 @@ import torch
 from gpu_helpers import bits_of, to_dev
 from helpers import oracle_compress
 from losslessly_compressed_tensors_b200.LCTensor import LCTTensor
+from losslessly_compressed_tensors_b200.codec import pointwise
+from losslessly_compressed_tensors_b200.codec.geometry import geometry
 from losslessly_compressed_tensors_b200.comp_format import Distribution, DistType, NoiseLevel
+from losslessly_compressed_tensors_b200.compression.huffman_tables import get_distribution_tables
+from losslessly_compressed_tensors_b200.kernels import dispatch
 from losslessly_compressed_tensors_b200.operations import (
     a_compA_add_B, a_compA_add_compB, compress, decompress, decompress_many,
 )
@@ -51,6 +55,35 @@ def test_walk(oracle, n, codebook, kind):
     dual = a_compA_add_compB(a, alpha, b)
     expect = oracle.pointwise(want_a, third, oracle.OP_SCALED, 0.95, alpha_is_one=False)
     assert np.array_equal(bits_of(dual).view(np.uint16), expect)
+
+
+def test_storage_with_more_than_2_31_elements_of_padding():
+    """Blocks of pure padding write nothing, also where their distance from the end of the tensor
+    does not fit 32 bits."""
+    n, guard, dist = 1000, 4096, CODEBOOKS["short"]
+    block_symbols, lanes, steps, fixed_words = geometry(dist)
+    blocks = (1 << 31) // block_symbols + 2
+    size = blocks * block_symbols
+    bits = synth_bf16(n, 11, "normal")
+    one = compress(to_dev(bits), dist, TensorBuffer(1 << 20))
+    encoded = torch.zeros(fixed_words * blocks * lanes + 4, dtype=torch.int32, device="cuda")
+    encoded[:-4].view(fixed_words, blocks * lanes)[:, :lanes] = one.data[:-4].view(fixed_words, lanes)
+    side = torch.zeros(size, dtype=torch.uint8, device="cuda")
+    side[:block_symbols] = one.sign_mantissa
+    operand = dispatch.make_operand(encoded, side, one.decode_table, one.center,
+                                    dispatch.pair_table_for(dist, encoded.device),
+                                    dispatch.fallback_tail_args(None))
+    _, _, rare_length = get_distribution_tables(dist, encoded.device)
+    shape = dict(logical_numel=n, block_symbols=block_symbols, lanes=lanes, steps=steps,
+                 fixed_words=fixed_words, rare_length=rare_length)
+    out = torch.full((n + guard,), 77, dtype=torch.int16, device="cuda")
+    dispatch.decode_kernel(operand, out, size, **shape)
+    assert np.array_equal(out[:n].cpu().numpy(), bits) and bool((out[n:] == 77).all())
+    zeros = torch.zeros(n, dtype=torch.bfloat16, device="cuda")
+    out = torch.full((n + guard,), 77, dtype=torch.int16, device="cuda")
+    dispatch.pointwise_dense(operand, zeros, out, None, size, None, None, op=pointwise.ADD.code,
+                             alpha_is_one=True, beta_is_one=True, compressed_output=False, **shape)
+    assert np.array_equal(out[:n].cpu().numpy(), bits) and bool((out[n:] == 77).all())
 
 
 @pytest.mark.parametrize("codebook", sorted(CODEBOOKS))
