@@ -59,9 +59,12 @@ struct BlockDecoder {
       }
       emit(kWalkPairs - 1);
     } else {
-      walk.read_chunk(step0, g.steps, [&](int k, uint32_t entry) {
-        out.store_guarded(word_at<kLaneMask>(offset, k, g.lane_mask),
-                          join_word(rows.exponents(entry, rows.neighbours(entry)), sides.pair(k)));
+      const bool full = out.holds_rows(step0 + kWalkRows);
+      walk.read_chunk(step0, [&](int k, uint32_t entry) {
+        const uint32_t at = word_at<kLaneMask>(offset, k, g.lane_mask);
+        const uint32_t word = join_word(rows.exponents(entry, rows.neighbours(entry)), sides.pair(k));
+        if (full) out.store(at, word);
+        else out.store_guarded(at, word);
       });
     }
   }
@@ -252,15 +255,25 @@ struct BlockPointwise {
       }
       emit_pair(kWalkPairs - 1);
     } else {
-      walk_a.read_chunk(step0, g.steps, [&](int k, uint32_t entry_a) {
+      int from_b = 0;
+      uint32_t tail_b[kWalkPairs / 2] = {};
+      if constexpr (kDual) {
+        from_b = walk_b.head->overflow_start[threadIdx.x];
+        walk_b.read_tail(tail_b, step0, from_b);
+      }
+      walk_a.read_chunk(step0, [&](int k, uint32_t entry_a) {
         const int step = step0 + 2 * k;
         uint32_t entry_b = 0u;
-        if constexpr (kDual) entry_b = walk_b.read_any(step, walk_b.tail_pair(step, g.steps));
+        if constexpr (kDual) {
+          if ((k & 1) == 0) walk_b.cursor.clamp();
+          entry_b = walk_b.read_any(step, from_b, (k & 1) ? tail_b[0] >> 8 : tail_b[0] << 8);
+          if (k & 1) next_word(tail_b);
+        }
         emit(step, word_at<kLaneMask>(offset, k, g.lane_mask), true,
              rows.exponents(entry_a, rows.neighbours(entry_a)),
              kDual ? rows.exponents(entry_b, rows.neighbours(entry_b)) : 0u, sides_a.pair(k),
              kDual ? sides_b.pair(k) : words[0]);
-        if (!kDual) next_pair(words);
+        if (!kDual) next_word(words);
       });
     }
   }

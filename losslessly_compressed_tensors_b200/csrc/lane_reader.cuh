@@ -174,6 +174,13 @@ __device__ __forceinline__ uint32_t look_up_entry(uint32_t table, uint32_t windo
   return entry;
 }
 
+// Move the word that was just used up out of a chunk's buffer.
+template <int kWords>
+__device__ __forceinline__ void next_word(uint32_t (&words)[kWords]) {
+#pragma unroll
+  for (int i = 0; i + 1 < kWords; ++i) words[i] = words[i + 1];
+}
+
 // The lane of one thread.  An entry that leaves this struct has the pair's exponent bytes in bytes
 // 1 and 2, whatever else is in it.
 struct LaneWalk {
@@ -232,42 +239,62 @@ struct LaneWalk {
     if (k & 1) cursor.refill();  // two full pairs take at most 24 bits: one refill serves both
     return entry;
   }
-  // Tail bytes of the pair at `step`, if it is in the tail (before the offset of 127).  Where the
-  // tail starts is read again each time: rarely needed, it would hold registers throughout.
-  __device__ __forceinline__ uint32_t tail_pair(int step, int steps) const {
-    const int from = head->overflow_start[threadIdx.x];
-    if (step < from || step >= steps) return 0u;
-    const uint8_t* t = head->tail + (head->overflow_offset[threadIdx.x] + step - from);
-    return (uint32_t)t[0] | ((uint32_t)t[1] << 16);
-  }
-  // The pair at `step`, wherever its symbols are; `raw`: tail_pair() of that step.
-  __device__ __forceinline__ uint32_t read_any(int step, uint32_t raw) {
-    if (step < coded) {
-      cursor.clamp();
-      const uint32_t before = cursor.lo;
-      uint32_t entry = look_up_entry(table, before);
-      if (step + 2 <= coded) {
-        cursor.take(entry);
-        if ((int32_t)entry < 0) entry = finish_pair(entry, before, false);
-      } else {  // the lane's last coded step is the first row of this pair
-        entry = ((entry & kEscape) ? literal(before) : entry_first_symbol(entry)) << 8;
-      }
-      cursor.refill();
-      return entry;
+  // Raw tail symbols of this lane in the rows from step0 on, four to a word, as exponent bytes
+  // (rows before the tail: undefined).  The tail is a run of bytes of any alignment: it is read in
+  // aligned words, each of which holds a byte of it, all of them requested together.
+  template <int kWords>
+  __device__ __forceinline__ void read_tail(uint32_t (&symbols)[kWords], int step0, int from) const {
+    const int index = step0 - from;  // of the first row, in the tail
+    uint32_t words[kWords + 1] = {};
+    int misaligned = 0;
+    if (index + 4 * kWords > 0) {
+      const uint8_t* first = head->tail + (head->overflow_offset[threadIdx.x] + index);
+      misaligned = (int)(reinterpret_cast<uintptr_t>(first) & 3u);
+      const uint32_t* aligned = reinterpret_cast<const uint32_t*>(first - misaligned);
+#pragma unroll
+      for (int i = 0; i <= kWords; ++i)
+        if (index + 4 * i + 3 >= misaligned && 4 * i < 4 * kWords + misaligned) words[i] = aligned[i];
     }
-    if (step < head->overflow_start[threadIdx.x]) return 0u;
-    return prmt(raw + 0x007F007Fu, 0u, 0x4204);  // bytes 0 and 2 to bytes 1 and 2
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) {
+      const uint32_t raw = __funnelshift_r(words[i], words[i + 1], 8 * misaligned);
+      symbols[i] = ((raw & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) ^ (raw & 0x80808080u);  // + 127, bytewise
+    }
+  }
+  // The pair at `step`, wherever its symbols are; `from`: where the lane's tail starts, `raw`: the
+  // entry the pair has if it is in the tail.
+  __device__ __forceinline__ uint32_t read_any(int step, int from, uint32_t raw) {
+    if (step >= coded) return step < from ? 0u : raw;
+    const uint32_t before = cursor.lo;
+    uint32_t entry = look_up_entry(table, before);
+    if (step + 2 <= coded) {
+      cursor.take(entry);
+      if ((int32_t)entry < 0) entry = finish_pair(entry, before, false);
+    } else {  // the lane's last coded step is the first row of this pair
+      entry = ((entry & kEscape) ? literal(before) : entry_first_symbol(entry)) << 8;
+    }
+    cursor.refill();
+    return entry;
   }
   // The pairs of a chunk in which some lane's stream ends, or has ended.  `emit(k, entry)` gets
-  // them one after the other; tail bytes are requested a pair ahead.
-  template <typename Emit>
-  __device__ __forceinline__ void read_chunk(int step0, int steps, Emit emit, int pairs = kWalkPairs) {
-    uint32_t ahead = tail_pair(step0, steps);
+  // them one after the other.  Where the tail starts is read again each time: it would hold a
+  // register throughout.  The tail's words are requested ahead of the loop; requested byte by byte
+  // inside it, each pair waits for global memory.  Two pairs per turn: unrolled over the chunk it
+  // saves 2 to 7 % here, and costs chunks of whole lanes as much or more (registers; decode.cu and
+  // update.cu, all codebooks).  Against the former pair-by-pair loop, 32 Mi elements that overflow
+  // in every lane: decoded in 176 -> 63 us (half-zero codebook), 99 -> 48 (normal codebook).
+  template <int kPairs = kWalkPairs, typename Emit>
+  __device__ __forceinline__ void read_chunk(int step0, Emit emit) {
+    constexpr int kWords = kPairs / 2;
+    const int from = head->overflow_start[threadIdx.x];
+    uint32_t symbols[kWords];
+    read_tail(symbols, step0, from);
 #pragma unroll 1
-    for (int k = 0; k < pairs; ++k) {
-      const uint32_t raw = ahead;
-      ahead = tail_pair(step0 + 2 * k + 2, steps);
-      emit(k, read_any(step0 + 2 * k, raw));
+    for (int k = 0; k < kPairs; k += 2) {
+      cursor.clamp();
+      emit(k, read_any(step0 + 2 * k, from, symbols[0] << 8));
+      emit(k + 1, read_any(step0 + 2 * k + 2, from, symbols[0] >> 8));
+      next_word(symbols);
     }
   }
 };
@@ -302,6 +329,8 @@ struct DenseWords {
   Element* rows;
   int left;  // elements_left()
 
+  // The first `count` rows of the block are full.
+  __device__ __forceinline__ bool holds_rows(int count) const { return count * kLanes <= left; }
   __device__ __forceinline__ void store(uint32_t at, uint32_t word) const {
     __stcs(reinterpret_cast<uint32_t*>(rows + at), word);
   }
@@ -316,13 +345,6 @@ struct DenseWords {
     return low | (high << 16);
   }
 };
-
-// Move the word of the pair that was just finished out of a chunk's buffer.
-template <int kPairs>
-__device__ __forceinline__ void next_pair(uint32_t (&words)[kPairs]) {
-#pragma unroll
-  for (int k = 0; k + 1 < kPairs; ++k) words[k] = words[k + 1];
-}
 
 // Rows of a block that hold elements, in whole chunks.
 __device__ __forceinline__ int rows_in_use(const Shape& g, int64_t block) {

@@ -585,7 +585,7 @@ struct BlockUpdate {
     const uint32_t offset = word_offset(row0, step0, g.lane_mask);
     const int valid = valid_steps_of(row0 / g.steps, threadIdx.x, g.steps, g.block_symbols,
                                      g.logical_numel, g.lane_mask);
-    walk.read_chunk(step0, g.steps, [&](int k, uint32_t entry) {
+    walk.read_chunk<kChunkPairs>(step0, [&](int k, uint32_t entry) {
       const int step = step0 + 2 * k;
       const uint32_t at = word_at<kLaneMask>(offset, k, g.lane_mask);
       const uint32_t result =
@@ -598,8 +598,8 @@ struct BlockUpdate {
       writer.append_checked(step < valid ? first : 0u, step + 1 < valid ? second : 0u, step,
                             (uint32_t)g.fixed_words * 32u);
       spill_pair<true>(at, exponents);
-      next_pair(right);
-    }, kChunkPairs);
+      next_word(right);
+    });
   }
   __device__ __forceinline__ void run() {
     Buffer now, next;

@@ -33,12 +33,27 @@ CODEBOOKS = {
 }
 
 
+KINDS = ["normal", "outliers", "wide", "staggered"]
+
+
+def values(n, seed, kind, base_exponent=0):
+    """``staggered``: every lane holds codable values up to a row of its own and incompressible
+    ones behind it, so the lanes of a warp leave their streams all over the block, and their tails
+    start at every alignment."""
+    if kind != "staggered":
+        return synth_bf16(n, seed, kind, base_exponent)
+    row, column = np.divmod(np.arange(n), 256)
+    lane = column ^ (row & 254)
+    wide = row % 128 >= (lane * 37 + seed) % 128
+    return np.where(wide, synth_bf16(n, seed, "wide"), synth_bf16(n, seed, "normal", base_exponent))
+
+
 @pytest.mark.parametrize("n", SIZES)
 @pytest.mark.parametrize("codebook", sorted(CODEBOOKS))
-@pytest.mark.parametrize("kind", ["normal", "outliers", "wide"])
+@pytest.mark.parametrize("kind", KINDS)
 def test_walk(oracle, n, codebook, kind):
     dist = CODEBOOKS[codebook]
-    bits, right, third = synth_bf16(n, 5, kind), synth_bf16(n + 1, 6, "normal", -2), synth_bf16(n, 7, kind)
+    bits, right, third = values(n, 5, kind), synth_bf16(n + 1, 6, "normal", -2), values(n, 7, kind)
     buffer = TensorBuffer(1 << 20)
     a, b = compress(to_dev(bits), dist, buffer), compress(to_dev(third), dist, buffer)
     assert np.array_equal(bits_of(decompress(a)), bits)
@@ -87,19 +102,19 @@ def test_storage_with_more_than_2_31_elements_of_padding():
 
 
 @pytest.mark.parametrize("codebook", sorted(CODEBOOKS))
-@pytest.mark.parametrize("kind", ["normal", "outliers", "wide"])
+@pytest.mark.parametrize("kind", KINDS)
 @pytest.mark.parametrize("offset", [0, 1])
 def test_batched_update_equals_single_updates(codebook, kind, offset):
     """The batched update walks lanes, the single one works on tiles: same payload, same result."""
     dist = CODEBOOKS[codebook]
     alpha = torch.tensor([0.95], dtype=torch.float32, device="cuda")
     buffer, reference = TensorBuffer(1 << 22), TensorBuffer(1 << 22)
-    bits = [synth_bf16(n, 20 + i, kind) for i, n in enumerate(SIZES)]
+    bits = [values(n, 20 + i, kind) for i, n in enumerate(SIZES)]
     together = [LCTTensor(to_dev(b), buffer, dist) for b in bits]
     alone = [LCTTensor(to_dev(b), reference, dist) for b in bits]
     plan = UpdatePlan(together, alpha)
     for step in range(3):
-        grads = [to_dev(synth_bf16(n + 1, 40 + 20 * step + i, kind, step - 1))[offset:offset + n]
+        grads = [to_dev(values(n + 1, 40 + 20 * step + i, kind, step - 1))[offset:offset + n]
                  for i, n in enumerate(SIZES)]
         plan.step(grads)
         for a, b, g in zip(together, alone, grads):
