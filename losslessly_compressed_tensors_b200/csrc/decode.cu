@@ -177,19 +177,20 @@ decode_batch_kernel(const lct_decode_job* __restrict__ jobs, int n_jobs, Shape c
 // One codec block, divided among threads as in the plain decoder.  The second operand is a dense
 // tensor (its words are requested ahead, like the side bytes) or, kDual, another compressed one,
 // whose lane the same thread walks.
-// `compressed`: the result leaves as side bytes (storage order) and exponent bytes (`auxiliary`,
+// kForm: the operation's arithmetic, a constant of the kernel (see Operation).
+// kCompressed: the result leaves as side bytes (storage order) and exponent bytes (`auxiliary`,
 // element order) instead of dense values; padding counts as +0.0.
-// Measured against the former tile form: 3072 x 4096 one compressed operand 41.0 -> 35.2 us, two
-// compressed operands and a compressed result (768 x 2304) 46.8 -> 35.8; 8192 x 4096 in blocks of
-// 32768 54.8 -> 56.9 (the one size found that lost).
-template <bool kDual, int kLaneMask>
+// Measured, a * A + B / A * B of one compressed operand, us (former tile form -> this): normal
+// codebook 32768 elements 14.8 -> 9.6 / 10.3 -> 8.9, 16 Mi 26.1 -> 22.9 / 21.6 -> 20.8, 64 Mi 89.8 ->
+// 72.5 / 74.9 -> 67.6; half-zero codebook 28 Mi 48.3 -> 41.4 / 40.6 -> 38.4; two compressed operands,
+// 12 Mi 44.3 -> 38.7.
+template <bool kDual, int kLaneMask, int kForm, bool kCompressed>
 struct BlockPointwise {
   const Shape& g;
-  Operation operation;
+  Operation<kForm> operation;
   int64_t row0;
   DenseWords<const uint16_t> other;
   int wide_rows;  // rows, in whole chunks, of `other` that may be read as words
-  bool compressed;
   DenseWords<uint16_t> out;  // dense result
   uint8_t* side_out;
   DenseWords<uint8_t> exponents_out;
@@ -213,7 +214,7 @@ struct BlockPointwise {
     const uint32_t left = join_word(exponents_a, from_a);
     const uint32_t right = kDual ? join_word(exponents_b, from_b) : from_b;
     uint32_t result = operation(left, right);
-    if (!compressed) {
+    if (!kCompressed) {
       if (guarded) out.store_guarded(at, result);
       else out.store(at, result);
       return;
@@ -255,6 +256,7 @@ struct BlockPointwise {
       }
       emit_pair(kWalkPairs - 1);
     } else {
+      const bool full = out.holds_rows(step0 + kWalkRows);
       int from_b = 0;
       uint32_t tail_b[kWalkPairs / 2] = {};
       if constexpr (kDual) {
@@ -269,7 +271,7 @@ struct BlockPointwise {
           entry_b = walk_b.read_any(step, from_b, (k & 1) ? tail_b[0] >> 8 : tail_b[0] << 8);
           if (k & 1) next_word(tail_b);
         }
-        emit(step, word_at<kLaneMask>(offset, k, g.lane_mask), true,
+        emit(step, word_at<kLaneMask>(offset, k, g.lane_mask), !full,
              rows.exponents(entry_a, rows.neighbours(entry_a)),
              kDual ? rows.exponents(entry_b, rows.neighbours(entry_b)) : 0u, sides_a.pair(k),
              kDual ? sides_b.pair(k) : words[0]);
@@ -279,13 +281,16 @@ struct BlockPointwise {
   }
 };
 
-constexpr int kPointwiseMinCtas = 3, kDualMinCtas = 2;
+// Resident CTAs per SM.  Dense results: four, although three are up to 8 % faster below 10 Mi
+// elements (no spills): with 444 slots a tensor of 448 to 592 blocks takes a second wave (28 Mi
+// half zeros, A * B: 42.2 us with three, 38.4 with four; the tile form took 40.6).  Compressed
+// results: three, 2 to 6 % faster than four throughout, the encoder behind included.
+constexpr int pointwise_ctas(bool dual, bool compressed) { return dual ? 2 : compressed ? 3 : 4; }
 
-template <bool kDual, int kLaneMask>
-__global__ void __launch_bounds__(kThreads, kDual ? kDualMinCtas : kPointwiseMinCtas)
+template <bool kDual, int kLaneMask, int kForm, bool kCompressed>
+__global__ void __launch_bounds__(kThreads, pointwise_ctas(kDual, kCompressed))
 pointwise_kernel(OperandView a, OperandView b, Shape g_in, const uint16_t* other,
-                 bool other_word_ok, void* output, uint8_t* auxiliary, OpSpec spec,
-                 bool compressed) {
+                 bool other_word_ok, void* output, uint8_t* auxiliary, OpSpec spec) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Shape g = g_in;
   if (kLaneMask >= 0) g.lane_mask = kLaneMask;  // see BlockDecoder
@@ -300,19 +305,20 @@ pointwise_kernel(OperandView a, OperandView b, Shape g_in, const uint16_t* other
   const int left = elements_left(g, block);
   const int rows_used = rows_in_use(g, block);
   uint8_t* side_out = static_cast<uint8_t*>(output) + block_base;
-  BlockPointwise<kDual, kLaneMask> work{
-      g, Operation(spec), block * g.steps, {other + (kDual ? 0 : block_base), left},
-      other_word_ok ? min(g.steps, left / kLanes) / kWalkRows * kWalkRows : 0, compressed,
-      {static_cast<uint16_t*>(output) + (compressed ? 0 : block_base), left},
-      side_out + own_bytes(), {auxiliary + (compressed ? block_base : 0), left}, rows_used, {}, {}, {},
+  using Block = BlockPointwise<kDual, kLaneMask, kForm, kCompressed>;
+  Block work{
+      g, Operation<kForm>(spec), block * g.steps, {other + (kDual ? 0 : block_base), left},
+      other_word_ok ? min(g.steps, left / kLanes) / kWalkRows * kWalkRows : 0,
+      {static_cast<uint16_t*>(output) + (kCompressed ? 0 : block_base), left},
+      side_out + own_bytes(), {auxiliary + (kCompressed ? block_base : 0), left}, rows_used, {}, {}, {},
       {}, {}};
-  typename BlockPointwise<kDual, kLaneMask>::Buffer now, next;
+  typename Block::Buffer now, next;
   work.request(now, 0);
   if (kDual) work.sides_b.open(rings + kRingBytes, b.side + block_base, rows_used);
   work.sides_a.open(rings, a.side + block_base, rows_used);
   stage_operand(sh, a, g, block);
   if (kDual) stage_operand(sh_b, b, g, block);
-  if (compressed)
+  if (kCompressed)
     for (int row = rows_used + (tid >> 6); row < g.steps; row += 4)
       reinterpret_cast<uint32_t*>(side_out + row * kLanes)[tid & 63] = 0u;
   work.rows.open();
@@ -330,6 +336,25 @@ pointwise_kernel(OperandView a, OperandView b, Shape g_in, const uint16_t* other
     if (kDual) work.sides_b.advance();
 #pragma unroll
     for (int k = 0; k < kWalkPairs; ++k) now[k] = next[k];
+  }
+}
+
+using PointwiseKernel = void (*)(OperandView, OperandView, Shape, const uint16_t*, bool, void*,
+                                uint8_t*, OpSpec);
+template <int kForm>
+static PointwiseKernel pointwise_kernel_of(bool swizzled, bool compressed) {
+  if (swizzled)
+    return compressed ? pointwise_kernel<false, 254, kForm, true> : pointwise_kernel<false, 254, kForm, false>;
+  return compressed ? pointwise_kernel<false, -1, kForm, true> : pointwise_kernel<false, -1, kForm, false>;
+}
+static PointwiseKernel pointwise_kernel_of(int form, bool swizzled, bool compressed) {
+  switch (form) {
+    case kFormLerp: return pointwise_kernel_of<kFormLerp>(swizzled, compressed);
+    case kFormRightScaled: return pointwise_kernel_of<kFormRightScaled>(swizzled, compressed);
+    case kFormAdd: return pointwise_kernel_of<kFormAdd>(swizzled, compressed);
+    case kFormMultiply: return pointwise_kernel_of<kFormMultiply>(swizzled, compressed);
+    case kFormEmaSquare: return pointwise_kernel_of<kFormEmaSquare>(swizzled, compressed);
+    default: return pointwise_kernel_of<kFormScaled>(swizzled, compressed);
   }
 }
 
@@ -387,11 +412,12 @@ int lct_pointwise(const lct_operand* a, const void* other, void* output, uint8_t
   if ((reinterpret_cast<uintptr_t>(other) & 1u) != 0) return LCT_E_ALIGNMENT;
   const lct::OpSpec spec{alpha, beta, op, alpha_is_one, beta_is_one};
   const size_t shared = lct::reader_shared_bytes(1, fixed_words, lct::kRingBytes);
-  auto kernel = g.lane_mask == 254 ? lct::pointwise_kernel<false, 254> : lct::pointwise_kernel<false, -1>;
+  auto kernel = lct::pointwise_kernel_of(lct::form_of(op, alpha_is_one, beta_is_one),
+                                         g.lane_mask == 254, compressed_output != 0);
   if ((rc = lct::opt_in_shared(kernel, shared)) != 0) return rc;
   kernel<<<(unsigned)g.n_blocks, lct::kThreads, shared, static_cast<cudaStream_t>(stream)>>>(
       va, va, g, static_cast<const uint16_t*>(other), (reinterpret_cast<uintptr_t>(other) & 3u) == 0, output, auxiliary,
-      spec, compressed_output != 0);
+      spec);
   return (int)cudaGetLastError();
 }
 
@@ -412,10 +438,15 @@ int lct_dual_scale_add(const lct_operand* a, const lct_operand* b, void* output,
   // fma(a, alpha, b): the scaled operation with beta == 1.
   const lct::OpSpec spec{alpha, nullptr, LCT_OP_SCALAR_MUL_ADD, 0, 1};
   const size_t shared = lct::reader_shared_bytes(2, fixed_words, 2 * lct::kRingBytes);
-  auto kernel = g.lane_mask == 254 ? lct::pointwise_kernel<true, 254> : lct::pointwise_kernel<true, -1>;
+  constexpr int kForm = lct::kFormScaled;
+  auto kernel = g.lane_mask == 254
+                    ? (compressed_output ? lct::pointwise_kernel<true, 254, kForm, true>
+                                         : lct::pointwise_kernel<true, 254, kForm, false>)
+                    : (compressed_output ? lct::pointwise_kernel<true, -1, kForm, true>
+                                         : lct::pointwise_kernel<true, -1, kForm, false>);
   if ((rc = lct::opt_in_shared(kernel, shared)) != 0) return rc;
   kernel<<<(unsigned)g.n_blocks, lct::kThreads, shared, static_cast<cudaStream_t>(stream)>>>(
-      va, vb, g, nullptr, false, output, auxiliary, spec, compressed_output != 0);
+      va, vb, g, nullptr, false, output, auxiliary, spec);
   return (int)cudaGetLastError();
 }
 

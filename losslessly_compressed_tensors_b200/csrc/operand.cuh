@@ -67,26 +67,17 @@ struct OpSpec {
 
 // The arithmetic forms behind the operations.  fma(l, alpha, r * beta) serves every scaled sum
 // but the one whose left operand is not scaled and whose right one is (it rounds once): a factor
-// of one changes neither the product nor the sum.  It comes first, so that the forms met most
-// cost one test per word.
+// of one changes neither the product nor the sum.
 enum OpForm { kFormScaled, kFormLerp, kFormRightScaled, kFormAdd, kFormMultiply, kFormEmaSquare };
 
-// An operation with its scalars, as a kernel applies it.
-struct Operation {
-  int form;
-  float alpha, beta;
-
-  __device__ __forceinline__ explicit Operation(const OpSpec& spec)
-      : alpha(spec.alpha_is_one ? 1.0f : *spec.alpha), beta(spec.beta_is_one ? 1.0f : *spec.beta) {
-    form = spec.op == LCT_OP_ADD          ? kFormAdd
-           : spec.op == LCT_OP_MULTIPLY   ? kFormMultiply
-           : spec.op == LCT_OP_LERP       ? kFormLerp
-           : spec.op == LCT_OP_EMA_SQUARE ? kFormEmaSquare
-           : spec.alpha_is_one && !spec.beta_is_one ? kFormRightScaled
-                                                    : kFormScaled;
-  }
-  __device__ __forceinline__ uint32_t operator()(uint32_t left, uint32_t right) const;
-};
+__host__ __device__ __forceinline__ int form_of(int op, int alpha_is_one, int beta_is_one) {
+  return op == LCT_OP_ADD          ? kFormAdd
+         : op == LCT_OP_MULTIPLY   ? kFormMultiply
+         : op == LCT_OP_LERP       ? kFormLerp
+         : op == LCT_OP_EMA_SQUARE ? kFormEmaSquare
+         : alpha_is_one && !beta_is_one ? kFormRightScaled
+                                        : kFormScaled;
+}
 
 __device__ __forceinline__ float bf16_low(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_high(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
@@ -109,27 +100,52 @@ __device__ __forceinline__ uint32_t lerp_pair(uint32_t start, uint32_t end, floa
 }
 
 // Two lanes of `left (op) right`, rounded once to BF16.
-__device__ __forceinline__ uint32_t Operation::operator()(uint32_t left, uint32_t right) const {
-  const float l0 = bf16_low(left), l1 = bf16_high(left);
-  const float r0 = bf16_low(right), r1 = bf16_high(right);
-  if (form == kFormScaled)
-    return pack_rn(__fmaf_rn(l0, alpha, __fmul_rn(r0, beta)), __fmaf_rn(l1, alpha, __fmul_rn(r1, beta)));
-  if (form == kFormLerp) return lerp_pair(left, right, alpha);
-  if (form == kFormRightScaled) return pack_rn(__fmaf_rn(r0, beta, l0), __fmaf_rn(r1, beta, l1));
-  if (form == kFormAdd) {
+template <int kForm>
+__device__ __forceinline__ uint32_t apply_form(uint32_t left, uint32_t right, float alpha, float beta) {
+  if (kForm == kFormAdd) {
     const __nv_bfloat162 r = __hadd2(*reinterpret_cast<const __nv_bfloat162*>(&left),
                                      *reinterpret_cast<const __nv_bfloat162*>(&right));
     return *reinterpret_cast<const uint32_t*>(&r);
   }
-  if (form == kFormMultiply) {
+  if (kForm == kFormMultiply) {
     const __nv_bfloat162 r = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&left),
                                      *reinterpret_cast<const __nv_bfloat162*>(&right));
     return *reinterpret_cast<const uint32_t*>(&r);
   }
-  const uint32_t scaled = pack_rn(__fmul_rn(l0, alpha), __fmul_rn(l1, alpha));
-  return pack_rn(__fmaf_rn(beta, __fmul_rn(r0, r0), bf16_low(scaled)),
-                 __fmaf_rn(beta, __fmul_rn(r1, r1), bf16_high(scaled)));
+  if (kForm == kFormLerp) return lerp_pair(left, right, alpha);
+  const float l0 = bf16_low(left), l1 = bf16_high(left);
+  const float r0 = bf16_low(right), r1 = bf16_high(right);
+  if (kForm == kFormRightScaled) return pack_rn(__fmaf_rn(r0, beta, l0), __fmaf_rn(r1, beta, l1));
+  if (kForm == kFormEmaSquare) {
+    const uint32_t scaled = pack_rn(__fmul_rn(l0, alpha), __fmul_rn(l1, alpha));
+    return pack_rn(__fmaf_rn(beta, __fmul_rn(r0, r0), bf16_low(scaled)),
+                   __fmaf_rn(beta, __fmul_rn(r1, r1), bf16_high(scaled)));
+  }
+  return pack_rn(__fmaf_rn(l0, alpha, __fmul_rn(r0, beta)), __fmaf_rn(l1, alpha, __fmul_rn(r1, beta)));
 }
+
+// An operation with its scalars.  The form is a constant of the kernel: tested per word, it cuts
+// the walk into pieces that no longer overlap (a product with a dense tensor took 15.0 instead of
+// 10.3 us for one block, 98.6 instead of 74.9 for 64 Mi elements).
+constexpr int kFormAtRunTime = -1;
+template <int kForm>
+struct Operation {
+  int form;
+  float alpha, beta;
+
+  __device__ __forceinline__ explicit Operation(const OpSpec& spec)
+      : form(form_of(spec.op, spec.alpha_is_one, spec.beta_is_one)),
+        alpha(spec.alpha_is_one ? 1.0f : *spec.alpha), beta(spec.beta_is_one ? 1.0f : *spec.beta) {}
+  __device__ __forceinline__ uint32_t operator()(uint32_t left, uint32_t right) const {
+    const int f = kForm == kFormAtRunTime ? form : kForm;
+    if (f == kFormScaled) return apply_form<kFormScaled>(left, right, alpha, beta);
+    if (f == kFormLerp) return apply_form<kFormLerp>(left, right, alpha, beta);
+    if (f == kFormRightScaled) return apply_form<kFormRightScaled>(left, right, alpha, beta);
+    if (f == kFormAdd) return apply_form<kFormAdd>(left, right, alpha, beta);
+    if (f == kFormMultiply) return apply_form<kFormMultiply>(left, right, alpha, beta);
+    return apply_form<kFormEmaSquare>(left, right, alpha, beta);
+  }
+};
 
 // ---------------------------------------------------------------------------
 // Host-side launch helpers

@@ -155,7 +155,7 @@ __device__ __forceinline__ void update_sample_chunk(const OperandView& a, const 
   // Same jittered position as the center estimate (one per equal slice of the tensor).
   const int64_t pos = sample_position(idx, n);
   const uint32_t right = other[pos];
-  const Operation operation(spec);
+  const Operation<kFormAtRunTime> operation(spec);
   uint32_t left;
   if (known != nullptr) {
     // A's values at the sample positions were kept when A was made: no stream to walk.
@@ -206,7 +206,7 @@ update_center_known_kernel(const uint16_t* __restrict__ other, int64_t n, OpSpec
                            int32_t* shifted_encode, int32_t* shifted_decode) {
   cudaTriggerProgrammaticLaunchCompletion();  // the fused kernel may start its prologue
   const int64_t count = n < kSampleCount ? n : kSampleCount;
-  const Operation operation(spec);
+  const Operation<kFormAtRunTime> operation(spec);
   int raw[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
@@ -485,7 +485,7 @@ static inline __host__ __device__ size_t update_walk_shared_bytes(int fixed_word
 template <int kLaneMask, int kEmit>
 struct BlockUpdate {
   const Shape& g;
-  Operation operation;
+  Operation<kFormAtRunTime> operation;
   int64_t row0;
   uint8_t* side_out;
   DenseWords<const uint16_t> other;
@@ -655,7 +655,7 @@ __device__ __forceinline__ void update_walk_block(
   // A job table comes from the caller's device memory: an unaligned by-product pointer takes
   // the scalar stores, a missing one is skipped.
   BlockUpdate<kLaneMask, kEmit> work{
-      g, Operation(spec), block * g.steps, side_out + block_base + own_bytes(),
+      g, Operation<kFormAtRunTime>(spec), block * g.steps, side_out + block_base + own_bytes(),
       {other + block_base, left}, word_ok ? min(g.steps, left / kLanes) / kChunkRows * kChunkRows : 0,
       {dense_out == nullptr ? nullptr : dense_out + block_base, left},
       (reinterpret_cast<uintptr_t>(dense_out) & 3u) == 0, spill + block_base, rows_used,

@@ -10,6 +10,7 @@ from gpu_helpers import bits_of, to_dev
 from helpers import oracle_compress
 from losslessly_compressed_tensors_b200.LCTensor import LCTTensor
 from losslessly_compressed_tensors_b200.codec import pointwise
+from losslessly_compressed_tensors_b200.codec.decode import operand_of
 from losslessly_compressed_tensors_b200.codec.geometry import geometry
 from losslessly_compressed_tensors_b200.comp_format import Distribution, DistType, NoiseLevel
 from losslessly_compressed_tensors_b200.compression.huffman_tables import get_distribution_tables
@@ -70,6 +71,34 @@ def test_walk(oracle, n, codebook, kind):
     dual = a_compA_add_compB(a, alpha, b)
     expect = oracle.pointwise(want_a, third, oracle.OP_SCALED, 0.95, alpha_is_one=False)
     assert np.array_equal(bits_of(dual).view(np.uint16), expect)
+
+
+@pytest.mark.parametrize("n", [CHUNK + 1, 65536 + 7 * CHUNK + 513])
+@pytest.mark.parametrize("op", ["LERP", "EMA_SQUARE"])
+def test_averages_of_one_compressed_operand(oracle, n, op):
+    """The two operations that the functional interface reaches through updates only."""
+    dist, alpha, beta = CODEBOOKS["short"], 0.25, 0.125
+    bits, right = values(n, 5, "staggered"), synth_bf16(n, 6, "normal", -2)
+    a = compress(to_dev(bits), dist, TensorBuffer(1 << 20))
+    want_a = oracle_compress(oracle, bits, dist, oracle.new_arena(1 << 20))
+    scalars = [torch.tensor([v], dtype=torch.float32, device="cuda") for v in (alpha, beta)]
+    block_symbols, lanes, steps, fixed_words = geometry(dist)
+    _, _, rare_length = get_distribution_tables(dist, a.data.device)
+    for dense in (True, False):
+        out = torch.empty(n if dense else a.size, dtype=torch.bfloat16 if dense else torch.uint8, device="cuda")
+        exponents = torch.zeros(a.size, dtype=torch.uint8, device="cuda")
+        dispatch.pointwise_dense(operand_of(a), to_dev(right), out, exponents, a.size, *scalars,
+                                 op=getattr(dispatch, "OP_" + op), alpha_is_one=False,
+                                 beta_is_one=False, compressed_output=not dense, logical_numel=n,
+                                 block_symbols=block_symbols, lanes=lanes, steps=steps,
+                                 fixed_words=fixed_words, rare_length=rare_length)
+        want = oracle.pointwise(want_a, right, getattr(oracle, "OP_" + op), alpha, beta,
+                                alpha_is_one=False, beta_is_one=False, dense=dense)
+        if dense:
+            assert np.array_equal(bits_of(out).view(np.uint16), want)
+        else:
+            assert np.array_equal(out.cpu().numpy(), want[0])
+            assert np.array_equal(exponents[:n].cpu().numpy(), want[1][:n])
 
 
 def test_storage_with_more_than_2_31_elements_of_padding():
