@@ -184,13 +184,19 @@ decode_batch_kernel(const lct_decode_job* __restrict__ jobs, int n_jobs, Shape c
 // codebook 32768 elements 14.8 -> 9.6 / 10.3 -> 8.9, 16 Mi 26.1 -> 22.9 / 21.6 -> 20.8, 64 Mi 89.8 ->
 // 72.5 / 74.9 -> 67.6; half-zero codebook 28 Mi 48.3 -> 41.4 / 40.6 -> 38.4; two compressed operands,
 // 12 Mi 44.3 -> 38.7.
-template <bool kDual, int kLaneMask, int kForm, bool kCompressed>
+// kAligned: the dense operand's words of two values are aligned.  Where they are not, a word is
+// two loads of two bytes, joined only when it is used (joined at once, the loads' latency would be
+// waited for), and a chunk's registers are requested again as they become free, half a chunk
+// ahead, in place of a second buffer.  a * A + B with B at an odd multiple of two bytes, normal
+// codebook, us (tile form -> guarded loads of single values -> this): 32768 elements 18.7 -> 18.6 ->
+// 11.8, 32 Mi 75 -> 87 -> 45, 64 Mi 140 -> 169 -> 87.
+template <bool kDual, int kLaneMask, int kForm, bool kCompressed, bool kAligned>
 struct BlockPointwise {
   const Shape& g;
   Operation<kForm> operation;
   int64_t row0;
   DenseWords<const uint16_t> other;
-  int wide_rows;  // rows, in whole chunks, of `other` that may be read as words
+  int wide_rows;  // rows, in whole chunks, of `other` that are full
   DenseWords<uint16_t> out;  // dense result
   uint8_t* side_out;
   DenseWords<uint8_t> exponents_out;
@@ -199,14 +205,30 @@ struct BlockPointwise {
   SideRing sides_a, sides_b;
   LaneWalk walk_a, walk_b;
 
-  using Buffer = uint32_t[kWalkPairs];
+  struct Buffer {
+    uint32_t word[kWalkPairs];  // or its first value
+    uint32_t second[kAligned ? 1 : kWalkPairs];
+
+    __device__ __forceinline__ uint32_t operator[](int k) const {
+      return kAligned ? word[k] : word[k] | (second[k] << 16);
+    }
+  };
+  template <int kFrom = 0, int kTo = kWalkPairs>
   __device__ __forceinline__ void request(Buffer& words, int step0) const {
     if (kDual || step0 >= rows_used) return;
     const uint32_t offset = word_offset(row0, step0, g.lane_mask);
 #pragma unroll
-    for (int k = 0; k < kWalkPairs; ++k) {
+    for (int k = kFrom; k < kTo; ++k) {
       const uint32_t at = word_at<kLaneMask>(offset, k, g.lane_mask);
-      words[k] = step0 < wide_rows ? other.load(at) : other.load_guarded(at);
+      if (kAligned) {
+        words.word[k] = step0 < wide_rows ? other.load(at) : other.load_guarded(at);
+      } else if (step0 < wide_rows) {
+        words.word[k] = other.load_value(at);
+        words.second[k] = other.load_value(at + 1);
+      } else {
+        words.word[k] = other.load_guarded(at);
+        words.second[k] = 0u;
+      }
     }
   }
   __device__ __forceinline__ void emit(int step, uint32_t at, bool guarded, uint32_t exponents_a,
@@ -245,6 +267,8 @@ struct BlockPointwise {
 #pragma unroll
       for (int k = 0; k < kWalkPairs; ++k) {
         const uint32_t next_a = walk_a.read_pair(k, [&] { if (k > 0) emit_pair(k - 1); });
+        if (!kAligned && k == kWalkPairs / 2)
+          request<0, kWalkPairs / 2>(words, step0 + kWalkRows);
         entry_a = next_a;
         neighbour_a = rows.neighbours(entry_a);
         side_a = sides_a.pair(k);
@@ -255,6 +279,7 @@ struct BlockPointwise {
         }
       }
       emit_pair(kWalkPairs - 1);
+      if (!kAligned) request<kWalkPairs / 2>(words, step0 + kWalkRows);
     } else {
       const bool full = out.holds_rows(step0 + kWalkRows);
       int from_b = 0;
@@ -275,8 +300,10 @@ struct BlockPointwise {
              rows.exponents(entry_a, rows.neighbours(entry_a)),
              kDual ? rows.exponents(entry_b, rows.neighbours(entry_b)) : 0u, sides_a.pair(k),
              kDual ? sides_b.pair(k) : words[0]);
-        if (!kDual) next_word(words);
+        if (!kDual) next_word(words.word);
+        if (!kAligned) next_word(words.second);
       });
+      if (!kAligned) request(words, step0 + kWalkRows);
     }
   }
 };
@@ -287,10 +314,10 @@ struct BlockPointwise {
 // results: three, 2 to 6 % faster than four throughout, the encoder behind included.
 constexpr int pointwise_ctas(bool dual, bool compressed) { return dual ? 2 : compressed ? 3 : 4; }
 
-template <bool kDual, int kLaneMask, int kForm, bool kCompressed>
+template <bool kDual, int kLaneMask, int kForm, bool kCompressed, bool kAligned>
 __global__ void __launch_bounds__(kThreads, pointwise_ctas(kDual, kCompressed))
-pointwise_kernel(OperandView a, OperandView b, Shape g_in, const uint16_t* other,
-                 bool other_word_ok, void* output, uint8_t* auxiliary, OpSpec spec) {
+pointwise_kernel(OperandView a, OperandView b, Shape g_in, const uint16_t* other, void* output,
+                 uint8_t* auxiliary, OpSpec spec) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Shape g = g_in;
   if (kLaneMask >= 0) g.lane_mask = kLaneMask;  // see BlockDecoder
@@ -305,10 +332,10 @@ pointwise_kernel(OperandView a, OperandView b, Shape g_in, const uint16_t* other
   const int left = elements_left(g, block);
   const int rows_used = rows_in_use(g, block);
   uint8_t* side_out = static_cast<uint8_t*>(output) + block_base;
-  using Block = BlockPointwise<kDual, kLaneMask, kForm, kCompressed>;
+  using Block = BlockPointwise<kDual, kLaneMask, kForm, kCompressed, kAligned>;
   Block work{
       g, Operation<kForm>(spec), block * g.steps, {other + (kDual ? 0 : block_base), left},
-      other_word_ok ? min(g.steps, left / kLanes) / kWalkRows * kWalkRows : 0,
+      min(g.steps, left / kLanes) / kWalkRows * kWalkRows,
       {static_cast<uint16_t*>(output) + (kCompressed ? 0 : block_base), left},
       side_out + own_bytes(), {auxiliary + (kCompressed ? block_base : 0), left}, rows_used, {}, {}, {},
       {}, {}};
@@ -328,33 +355,34 @@ pointwise_kernel(OperandView a, OperandView b, Shape g_in, const uint16_t* other
   if (kDual) work.walk_b.open(sh_b, b, g, block);
 #pragma unroll 1
   for (int step0 = 0; step0 < rows_used; step0 += kWalkRows) {
-    work.request(next, step0 + kWalkRows);
+    if (kAligned) work.request(next, step0 + kWalkRows);
     if (kDual) work.sides_b.wait_both(work.sides_a);
     else work.sides_a.wait();
     work.chunk(step0, now);
     work.sides_a.advance();
     if (kDual) work.sides_b.advance();
-#pragma unroll
-    for (int k = 0; k < kWalkPairs; ++k) now[k] = next[k];
+    if (kAligned) now = next;
   }
 }
 
-using PointwiseKernel = void (*)(OperandView, OperandView, Shape, const uint16_t*, bool, void*,
-                                uint8_t*, OpSpec);
-template <int kForm>
-static PointwiseKernel pointwise_kernel_of(bool swizzled, bool compressed) {
-  if (swizzled)
-    return compressed ? pointwise_kernel<false, 254, kForm, true> : pointwise_kernel<false, 254, kForm, false>;
-  return compressed ? pointwise_kernel<false, -1, kForm, true> : pointwise_kernel<false, -1, kForm, false>;
+using PointwiseKernel = void (*)(OperandView, OperandView, Shape, const uint16_t*, void*, uint8_t*,
+                                OpSpec);
+// (Unaligned dense operands are rare: one kernel for both lane mappings serves them.)
+template <int kForm, bool kCompressed>
+static PointwiseKernel pointwise_kernel_of(bool swizzled, bool aligned) {
+  if (!aligned) return pointwise_kernel<false, -1, kForm, kCompressed, false>;
+  return swizzled ? pointwise_kernel<false, 254, kForm, kCompressed, true>
+                  : pointwise_kernel<false, -1, kForm, kCompressed, true>;
 }
-static PointwiseKernel pointwise_kernel_of(int form, bool swizzled, bool compressed) {
+template <bool kCompressed>
+static PointwiseKernel pointwise_kernel_of(int form, bool swizzled, bool aligned) {
   switch (form) {
-    case kFormLerp: return pointwise_kernel_of<kFormLerp>(swizzled, compressed);
-    case kFormRightScaled: return pointwise_kernel_of<kFormRightScaled>(swizzled, compressed);
-    case kFormAdd: return pointwise_kernel_of<kFormAdd>(swizzled, compressed);
-    case kFormMultiply: return pointwise_kernel_of<kFormMultiply>(swizzled, compressed);
-    case kFormEmaSquare: return pointwise_kernel_of<kFormEmaSquare>(swizzled, compressed);
-    default: return pointwise_kernel_of<kFormScaled>(swizzled, compressed);
+    case kFormLerp: return pointwise_kernel_of<kFormLerp, kCompressed>(swizzled, aligned);
+    case kFormRightScaled: return pointwise_kernel_of<kFormRightScaled, kCompressed>(swizzled, aligned);
+    case kFormAdd: return pointwise_kernel_of<kFormAdd, kCompressed>(swizzled, aligned);
+    case kFormMultiply: return pointwise_kernel_of<kFormMultiply, kCompressed>(swizzled, aligned);
+    case kFormEmaSquare: return pointwise_kernel_of<kFormEmaSquare, kCompressed>(swizzled, aligned);
+    default: return pointwise_kernel_of<kFormScaled, kCompressed>(swizzled, aligned);
   }
 }
 
@@ -412,12 +440,13 @@ int lct_pointwise(const lct_operand* a, const void* other, void* output, uint8_t
   if ((reinterpret_cast<uintptr_t>(other) & 1u) != 0) return LCT_E_ALIGNMENT;
   const lct::OpSpec spec{alpha, beta, op, alpha_is_one, beta_is_one};
   const size_t shared = lct::reader_shared_bytes(1, fixed_words, lct::kRingBytes);
-  auto kernel = lct::pointwise_kernel_of(lct::form_of(op, alpha_is_one, beta_is_one),
-                                         g.lane_mask == 254, compressed_output != 0);
+  const int form = lct::form_of(op, alpha_is_one, beta_is_one);
+  const bool swizzled = g.lane_mask == 254, aligned = (reinterpret_cast<uintptr_t>(other) & 3u) == 0;
+  auto kernel = compressed_output ? lct::pointwise_kernel_of<true>(form, swizzled, aligned)
+                                  : lct::pointwise_kernel_of<false>(form, swizzled, aligned);
   if ((rc = lct::opt_in_shared(kernel, shared)) != 0) return rc;
   kernel<<<(unsigned)g.n_blocks, lct::kThreads, shared, static_cast<cudaStream_t>(stream)>>>(
-      va, va, g, static_cast<const uint16_t*>(other), (reinterpret_cast<uintptr_t>(other) & 3u) == 0, output, auxiliary,
-      spec);
+      va, va, g, static_cast<const uint16_t*>(other), output, auxiliary, spec);
   return (int)cudaGetLastError();
 }
 
@@ -440,13 +469,13 @@ int lct_dual_scale_add(const lct_operand* a, const lct_operand* b, void* output,
   const size_t shared = lct::reader_shared_bytes(2, fixed_words, 2 * lct::kRingBytes);
   constexpr int kForm = lct::kFormScaled;
   auto kernel = g.lane_mask == 254
-                    ? (compressed_output ? lct::pointwise_kernel<true, 254, kForm, true>
-                                         : lct::pointwise_kernel<true, 254, kForm, false>)
-                    : (compressed_output ? lct::pointwise_kernel<true, -1, kForm, true>
-                                         : lct::pointwise_kernel<true, -1, kForm, false>);
+                    ? (compressed_output ? lct::pointwise_kernel<true, 254, kForm, true, true>
+                                         : lct::pointwise_kernel<true, 254, kForm, false, true>)
+                    : (compressed_output ? lct::pointwise_kernel<true, -1, kForm, true, true>
+                                         : lct::pointwise_kernel<true, -1, kForm, false, true>);
   if ((rc = lct::opt_in_shared(kernel, shared)) != 0) return rc;
   kernel<<<(unsigned)g.n_blocks, lct::kThreads, shared, static_cast<cudaStream_t>(stream)>>>(
-      va, vb, g, nullptr, false, output, auxiliary, spec);
+      va, vb, g, nullptr, output, auxiliary, spec);
   return (int)cudaGetLastError();
 }
 

@@ -339,6 +339,7 @@ struct DenseWords {
     if ((int)at + 1 < left) rows[at + 1] = (uint16_t)(word >> 16);
   }
   __device__ __forceinline__ uint32_t load(uint32_t at) const { return load_ahead_u32(rows + at); }
+  __device__ __forceinline__ uint32_t load_value(uint32_t at) const { return load_ahead_u16(rows + at); }
   __device__ __forceinline__ uint32_t load_guarded(uint32_t at) const {
     const uint32_t low = (int)at < left ? rows[at] : 0u;
     const uint32_t high = (int)at + 1 < left ? rows[at + 1] : 0u;

@@ -75,10 +75,13 @@ def test_walk(oracle, n, codebook, kind):
 
 @pytest.mark.parametrize("n", [CHUNK + 1, 65536 + 7 * CHUNK + 513])
 @pytest.mark.parametrize("op", ["LERP", "EMA_SQUARE"])
-def test_averages_of_one_compressed_operand(oracle, n, op):
-    """The two operations that the functional interface reaches through updates only."""
+@pytest.mark.parametrize("offset", [0, 1])  # the dense operand at 16 and at 2 bytes alignment
+def test_averages_of_one_compressed_operand(oracle, n, op, offset):
+    """The two operations that the functional interface reaches through updates only, with dense
+    and with compressed results."""
     dist, alpha, beta = CODEBOOKS["short"], 0.25, 0.125
-    bits, right = values(n, 5, "staggered"), synth_bf16(n, 6, "normal", -2)
+    bits, wide = values(n, 5, "staggered"), synth_bf16(n + 1, 6, "normal", -2)
+    right, other = wide[offset:offset + n], to_dev(wide)[offset:offset + n]
     a = compress(to_dev(bits), dist, TensorBuffer(1 << 20))
     want_a = oracle_compress(oracle, bits, dist, oracle.new_arena(1 << 20))
     scalars = [torch.tensor([v], dtype=torch.float32, device="cuda") for v in (alpha, beta)]
@@ -87,7 +90,7 @@ def test_averages_of_one_compressed_operand(oracle, n, op):
     for dense in (True, False):
         out = torch.empty(n if dense else a.size, dtype=torch.bfloat16 if dense else torch.uint8, device="cuda")
         exponents = torch.zeros(a.size, dtype=torch.uint8, device="cuda")
-        dispatch.pointwise_dense(operand_of(a), to_dev(right), out, exponents, a.size, *scalars,
+        dispatch.pointwise_dense(operand_of(a), other, out, exponents, a.size, *scalars,
                                  op=getattr(dispatch, "OP_" + op), alpha_is_one=False,
                                  beta_is_one=False, compressed_output=not dense, logical_numel=n,
                                  block_symbols=block_symbols, lanes=lanes, steps=steps,
