@@ -463,10 +463,12 @@ update_fused_kernel(OperandView a, Shape g, const uint16_t* other, bool other_ve
 // Form of the batched update: a thread walks its lane (lane_reader.cuh) and appends to its own
 // output stream; neighbouring threads exchange exponents by shuffle on the way to their rows and
 // back.  Fewer instructions per pair than the tile form, but more registers, which leaves three
-// CTAs per SM instead of four (at four, spilling, all of the gain is lost).  Lists of tensors
-// fill the device several times over and gain: 12 x 4096 x 4096 444 -> 400 us, the 8 matrices of
-// two 768-wide layers 53.4 -> 49.7.  A single tensor of 400 to 600 blocks is one wave of the tile
-// form and loses (4096 x 4096 51.9 -> 52.7 us, 8192 x 4096 87.8 -> 92.1): it keeps that form.
+// CTAs per SM instead of four (at four, spilling, it is 10 to 45 % slower).  kForm: the operation's
+// arithmetic, a constant of the kernel (see Operation).
+//
+// A call, us (tile form -> operation tested per word -> this): 12 tensors of 4096 x 4096, normal
+// codebook 517 -> 530 -> 473; two of them 107 -> 116 -> 106; with the average and its look-ahead
+// direction 140 -> 156 -> 143; twelve of 100001 elements 57 -> 58 -> 50.
 
 // Shared memory of a CTA: [decode table | encode table, scan scratch, ring of side bytes | head,
 // input image].
@@ -482,10 +484,10 @@ static inline __host__ __device__ size_t update_walk_shared_bytes(int fixed_word
 // One thread of a block: its lane's walk and its lane's output stream, and between them its row of
 // every pair (two neighbouring columns, see lanes.cuh): join, operation, split.  Chunks of 8 rows,
 // half a stage of the ring.
-template <int kLaneMask, int kEmit>
+template <int kLaneMask, int kEmit, int kForm>
 struct BlockUpdate {
   const Shape& g;
-  Operation<kFormAtRunTime> operation;
+  Operation<kForm> operation;
   int64_t row0;
   uint8_t* side_out;
   DenseWords<const uint16_t> other;
@@ -621,7 +623,7 @@ struct BlockUpdate {
 };
 
 // One codec block of a batch; parameters as for update_fused_block.
-template <int kLaneMask, int kEmit>
+template <int kLaneMask, int kEmit, int kForm>
 __device__ __forceinline__ void update_walk_block(
     const OperandView& view, const Shape& g_in, const uint16_t* other, const OpSpec& spec,
     const int32_t* shifted_encode, uint8_t* side_out, uint32_t* encoded_out, uint8_t* extra_starts,
@@ -654,8 +656,8 @@ __device__ __forceinline__ void update_walk_block(
   const bool word_ok = (reinterpret_cast<uintptr_t>(other) & 3u) == 0;
   // A job table comes from the caller's device memory: an unaligned by-product pointer takes
   // the scalar stores, a missing one is skipped.
-  BlockUpdate<kLaneMask, kEmit> work{
-      g, Operation<kFormAtRunTime>(spec), block * g.steps, side_out + block_base + own_bytes(),
+  BlockUpdate<kLaneMask, kEmit, kForm> work{
+      g, Operation<kForm>(spec), block * g.steps, side_out + block_base + own_bytes(),
       {other + block_base, left}, word_ok ? min(g.steps, left / kLanes) / kChunkRows * kChunkRows : 0,
       {dense_out == nullptr ? nullptr : dense_out + block_base, left},
       (reinterpret_cast<uintptr_t>(dense_out) & 3u) == 0, spill + block_base, rows_used,
@@ -673,7 +675,7 @@ __device__ __forceinline__ void update_walk_block(
 constexpr int kUpdateWalkMinCtas = 3;
 
 // Every block of every job of a batch: CTA b serves the job whose block range contains b.
-template <int kLaneMask, int kEmit>
+template <int kLaneMask, int kEmit, int kForm>
 __global__ void __launch_bounds__(kThreads, kUpdateWalkMinCtas)
 update_fused_batch_kernel(const lct_update_job* __restrict__ jobs, int n_jobs, Shape common,
                           OpSpec spec, const int32_t* shifted_encode,
@@ -685,12 +687,30 @@ update_fused_batch_kernel(const lct_update_job* __restrict__ jobs, int n_jobs, S
     if (jobs[mid].first_block <= block) lo = mid; else hi = mid - 1;
   }
   const lct_update_job& job = jobs[lo];
-  update_walk_block<kLaneMask, kEmit>(
+  update_walk_block<kLaneMask, kEmit, kForm>(
       view_of_update(job.a), shape_of_update(job, common), static_cast<const uint16_t*>(job.other),
       spec, shifted_encode + 256 * (int64_t)lo, job.side_out,
       reinterpret_cast<uint32_t*>(job.encoded_out), extra_starts + job.first_block * kLanes,
       summaries + 4 * job.first_block, job.spill, static_cast<uint16_t*>(job.dense_out),
       block - job.first_block);
+}
+
+using UpdateBatchKernel = void (*)(const lct_update_job*, int, Shape, OpSpec, const int32_t*,
+                                   uint8_t*, int32_t*);
+template <int kEmit, int kForm>
+static UpdateBatchKernel update_batch_kernel_of(bool swizzled) {
+  return swizzled ? update_fused_batch_kernel<254, kEmit, kForm> : update_fused_batch_kernel<-1, kEmit, kForm>;
+}
+template <int kEmit>
+static UpdateBatchKernel update_batch_kernel_of(int form, bool swizzled) {
+  switch (form) {
+    case kFormLerp: return update_batch_kernel_of<kEmit, kFormLerp>(swizzled);
+    case kFormRightScaled: return update_batch_kernel_of<kEmit, kFormRightScaled>(swizzled);
+    case kFormAdd: return update_batch_kernel_of<kEmit, kFormAdd>(swizzled);
+    case kFormMultiply: return update_batch_kernel_of<kEmit, kFormMultiply>(swizzled);
+    case kFormEmaSquare: return update_batch_kernel_of<kEmit, kFormEmaSquare>(swizzled);
+    default: return update_batch_kernel_of<kEmit, kFormScaled>(swizzled);
+  }
 }
 
 }  // namespace lct
@@ -913,14 +933,11 @@ int lct_update_batch_emit(const lct_update_job* jobs, int n_jobs, int64_t total_
   if (emit < LCT_EMIT_NONE || emit > LCT_EMIT_NESTEROV) return LCT_E_BAD_ARGUMENT;
   if (emit == LCT_EMIT_NESTEROV && (op != LCT_OP_LERP || beta == nullptr)) return LCT_E_BAD_ARGUMENT;
   const bool swizzled = g.lane_mask == 254;
+  const int form = lct::form_of(op, alpha_is_one, beta_is_one);
   auto kernel = emit == LCT_EMIT_NESTEROV
-                    ? (swizzled ? lct::update_fused_batch_kernel<254, LCT_EMIT_NESTEROV>
-                                : lct::update_fused_batch_kernel<-1, LCT_EMIT_NESTEROV>)
-                : emit == LCT_EMIT_RESULT
-                    ? (swizzled ? lct::update_fused_batch_kernel<254, LCT_EMIT_RESULT>
-                                : lct::update_fused_batch_kernel<-1, LCT_EMIT_RESULT>)
-                    : (swizzled ? lct::update_fused_batch_kernel<254, LCT_EMIT_NONE>
-                                : lct::update_fused_batch_kernel<-1, LCT_EMIT_NONE>);
+                    ? lct::update_batch_kernel_of<LCT_EMIT_NESTEROV, lct::kFormLerp>(swizzled)
+                : emit == LCT_EMIT_RESULT ? lct::update_batch_kernel_of<LCT_EMIT_RESULT>(form, swizzled)
+                                          : lct::update_batch_kernel_of<LCT_EMIT_NONE>(form, swizzled);
   if ((rc = lct::opt_in_shared(kernel, shared)) != 0) return rc;
   if ((rc = lct::launch_overlapped(kernel, (unsigned)total_blocks, lct::kThreads, shared, st, jobs,
                                    n_jobs, g, spec, shifted_encode, extra_starts, summaries)))

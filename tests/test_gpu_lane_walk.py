@@ -8,6 +8,7 @@ import torch
 
 from gpu_helpers import bits_of, to_dev
 from helpers import oracle_compress
+from losslessly_compressed_tensors_b200 import config
 from losslessly_compressed_tensors_b200.LCTensor import LCTTensor
 from losslessly_compressed_tensors_b200.codec import pointwise
 from losslessly_compressed_tensors_b200.codec.decode import operand_of
@@ -131,6 +132,66 @@ def test_storage_with_more_than_2_31_elements_of_padding():
     dispatch.pointwise_dense(operand, zeros, out, None, size, None, None, op=pointwise.ADD.code,
                              alpha_is_one=True, beta_is_one=True, compressed_output=False, **shape)
     assert np.array_equal(out[:n].cpu().numpy(), bits) and bool((out[n:] == 77).all())
+
+
+@pytest.fixture(params=["swizzle", "linear"])
+def lane_mapping(request, monkeypatch):
+    monkeypatch.setattr(config, "lane_mapping", request.param)
+    yield request.param
+    monkeypatch.undo()
+    # hand the default mapping back to the library before any other test launches
+    x = torch.zeros(256, dtype=torch.bfloat16, device="cuda")
+    assert torch.equal(decompress(compress(x, CODEBOOKS["short"])), x)
+
+
+NONE, RESULT, NESTEROV = dispatch.EMIT_NONE, dispatch.EMIT_RESULT, dispatch.EMIT_NESTEROV
+# name: operation, its arguments, by-product
+FORMS = {
+    "scaled": (pointwise.SCALAR_MUL_ADD, dict(alpha=0.95), NONE),
+    "both scaled": (pointwise.SCALAR_MUL_ADD, dict(alpha=0.95, beta=0.3), RESULT),
+    "sum": (pointwise.SCALAR_MUL_ADD, dict(alpha=7.0, alpha_is_one=True), NONE),
+    "right scaled": (pointwise.SCALAR_MUL_ADD, dict(alpha=7.0, beta=0.3, alpha_is_one=True), NONE),
+    "add": (pointwise.ADD, dict(alpha=7.0), NONE),
+    "multiply": (pointwise.MULTIPLY, dict(alpha=7.0), RESULT),
+    "lerp": (pointwise.LERP, dict(alpha=0.05), RESULT),
+    "lerp, direction": (pointwise.LERP, dict(alpha=0.05, beta=0.95), NESTEROV),
+    "average of squares": (pointwise.EMA_SQUARE, dict(alpha=0.95, beta=0.05), RESULT),
+}
+
+
+@pytest.mark.parametrize("form", sorted(FORMS))
+@pytest.mark.parametrize("codebook", ["short", "long"])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_batched_update_forms_equal_single_updates(lane_mapping, form, codebook, offset):
+    """Every arithmetic form and by-product of the batched update, in both lane mappings, against
+    the single update: same payload, same result, same by-product (written over the update itself
+    where that is aligned)."""
+    operation, arguments, emit = FORMS[form]
+    arguments = {k: torch.tensor([v], dtype=torch.float32, device="cuda") if isinstance(v, float) else v
+                 for k, v in arguments.items()}
+    dist, sizes = CODEBOOKS[codebook], SIZES[2:]
+    buffer, reference = TensorBuffer(1 << 22), TensorBuffer(1 << 22)
+    bits = [values(n, 20 + i, "staggered") for i, n in enumerate(sizes)]
+    together = [LCTTensor(to_dev(b), buffer, dist) for b in bits]
+    alone = [LCTTensor(to_dev(b), reference, dist) for b in bits]
+    plan = UpdatePlan(together, operation=operation, emit=emit, **arguments)
+    for step in range(2):
+        wide = [to_dev(values(n + 1, 40 + 20 * step + i, "staggered", step - 1)) for i, n in enumerate(sizes)]
+        grads = [w[offset:offset + n] for w, n in zip(wide, sizes)]
+        expected = [torch.zeros(n, dtype=torch.bfloat16, device="cuda") for n in sizes]
+        for b, g, out in zip(alone, grads, expected):
+            new = pointwise.recycled_update(b.x, g, operation, emit=emit,
+                                            dense_out=out if emit != NONE else None, **arguments)
+            assert new is not None
+            b.x = new
+        outs = grads if offset == 0 else [torch.zeros_like(out) for out in expected]
+        plan.step(grads, outs if emit != NONE else None)
+        for a, b, out, want in zip(together, alone, outs, expected):
+            for part in ("data", "sign_mantissa", "center", "fallback_count"):
+                assert torch.equal(getattr(a.x, part), getattr(b.x, part)), (part, out.numel(), step)
+            assert torch.equal(decompress(a.x).view(torch.int16), decompress(b.x).view(torch.int16))
+            if emit != NONE:
+                assert torch.equal(out.view(torch.int16), want.view(torch.int16)), (out.numel(), step)
 
 
 @pytest.mark.parametrize("codebook", sorted(CODEBOOKS))
