@@ -24,6 +24,8 @@
 // exponents from the overflow step on into `spill` (logical order), which is
 // what the tail compaction reads afterwards; nothing else touches `spill`.
 #include "batch.cuh"
+#include <type_traits>
+
 #include "center.cuh"
 #include "decode_core.cuh"
 #include "encode_core.cuh"
@@ -467,8 +469,10 @@ update_fused_kernel(OperandView a, Shape g, const uint16_t* other, bool other_ve
 // arithmetic, a constant of the kernel (see Operation).
 //
 // A call, us (tile form -> operation tested per word -> this): 12 tensors of 4096 x 4096, normal
-// codebook 517 -> 530 -> 473; two of them 107 -> 116 -> 106; with the average and its look-ahead
-// direction 140 -> 156 -> 143; twelve of 100001 elements 57 -> 58 -> 50.
+// codebook 517 -> 530 -> 481; two of them 107 -> 116 -> 107; with the average and its look-ahead
+// direction 140 -> 156 -> 140; twelve of 100001 elements 57 -> 58 -> 50; two with the dense operand
+// at an odd multiple of two bytes 130 -> 191 -> 107.  (The code for such operands costs the aligned
+// ones 1 to 3 %: it shares their register allocation.)
 
 // Shared memory of a CTA: [decode table | encode table, scan scratch, ring of side bytes | head,
 // input image].
@@ -483,17 +487,16 @@ static inline __host__ __device__ size_t update_walk_shared_bytes(int fixed_word
 
 // One thread of a block: its lane's walk and its lane's output stream, and between them its row of
 // every pair (two neighbouring columns, see lanes.cuh): join, operation, split.  Chunks of 8 rows,
-// half a stage of the ring.
-template <int kLaneMask, int kEmit, int kForm>
+// half a stage of the ring.  kAligned: the words of `other` and of the by-product are aligned.
+template <int kLaneMask, int kEmit, int kForm, bool kAligned>
 struct BlockUpdate {
   const Shape& g;
   Operation<kForm> operation;
   int64_t row0;
   uint8_t* side_out;
   DenseWords<const uint16_t> other;
-  int wide_rows;  // rows, in whole chunks, of `other` that may be read as words
+  int wide_rows;  // rows, in whole chunks, of `other` that are full
   DenseWords<uint16_t> dense;  // kEmit: the dense by-product (may alias `other`)
-  bool dense_word_ok;
   uint8_t* spill;  // the block's first element
   int rows_used;
   uint32_t encode_table;
@@ -504,13 +507,32 @@ struct BlockUpdate {
   GlobalLaneWriter writer;
 
   using Buffer = uint32_t[kChunkPairs];  // words of `other`
-  __device__ __forceinline__ void request(Buffer& right, int step0) const {
+  // ... as they are requested a chunk ahead: unaligned ones in two halves, joined when the chunk's
+  // turn comes (joined at once, their latency would be waited for).
+  struct Requested {
+    Buffer word;
+    uint32_t second[kAligned ? 1 : kChunkPairs];
+
+    __device__ __forceinline__ void join(Buffer& words) const {
+#pragma unroll
+      for (int k = 0; k < kChunkPairs; ++k) words[k] = kAligned ? word[k] : word[k] | (second[k] << 16);
+    }
+  };
+  __device__ __forceinline__ void request(Requested& right, int step0) const {
     if (step0 >= rows_used) return;
     const uint32_t offset = word_offset(row0, step0, g.lane_mask);
 #pragma unroll
     for (int k = 0; k < kChunkPairs; ++k) {
       const uint32_t at = word_at<kLaneMask>(offset, k, g.lane_mask);
-      right[k] = step0 < wide_rows ? other.load(at) : other.load_guarded(at);
+      if (kAligned) {
+        right.word[k] = step0 < wide_rows ? other.load(at) : other.load_guarded(at);
+      } else if (step0 < wide_rows) {
+        right.word[k] = other.load_value(at);
+        right.second[k] = other.load_value(at + 1);
+      } else {
+        right.word[k] = other.load_guarded(at);
+        right.second[k] = 0u;
+      }
     }
   }
   // This thread's row of the pair at `step`: its two result exponents (bytes 0 and 1).
@@ -522,11 +544,11 @@ struct BlockUpdate {
       if ((int)at >= other.left) result = 0u;
       else if ((int)at + 1 >= other.left) result &= 0xFFFFu;
     }
-    if (kEmit != LCT_EMIT_NONE && dense.rows != nullptr) {
+    if (kEmit != LCT_EMIT_NONE) {
       const uint32_t word =
           kEmit == LCT_EMIT_NESTEROV ? lerp_pair(right, result, operation.beta) : result;
-      if (!kGuarded && dense_word_ok) dense.store(at, word);
-      else dense.store_guarded(at, word);
+      if (kAligned && !kGuarded) dense.store(at, word);
+      else if (kAligned || dense.rows != nullptr) dense.store_guarded(at, word);
     }
     uint32_t sides_of_row, exponents;
     split_words(result, 0u, &sides_of_row, &exponents);
@@ -604,11 +626,13 @@ struct BlockUpdate {
     });
   }
   __device__ __forceinline__ void run() {
-    Buffer now, next;
-    request(now, 0);
+    Requested next;
+    request(next, 0);
 #pragma unroll 1
     for (int step0 = 0; step0 < rows_used; step0 += kChunkRows) {
       const int first_pair = (step0 & (kWalkRows - 1)) >> 1;
+      Buffer now;
+      next.join(now);
       request(next, step0 + kChunkRows);
       if (first_pair == 0) sides.wait();
       const bool far = writer.bits() + kChunkBits <= (uint32_t)g.fixed_words * 32u;
@@ -616,14 +640,12 @@ struct BlockUpdate {
       else if (__all_sync(0xFFFFFFFFu, far)) whole_chunk<false>(step0, first_pair, now);
       else whole_chunk<true>(step0, first_pair, now);
       if (first_pair != 0) sides.advance();
-#pragma unroll
-      for (int k = 0; k < kChunkPairs; ++k) now[k] = next[k];
     }
   }
 };
 
 // One codec block of a batch; parameters as for update_fused_block.
-template <int kLaneMask, int kEmit, int kForm>
+template <int kLaneMask, int kEmit, int kForm, bool kAligned>
 __device__ __forceinline__ void update_walk_block(
     const OperandView& view, const Shape& g_in, const uint16_t* other, const OpSpec& spec,
     const int32_t* shifted_encode, uint8_t* side_out, uint32_t* encoded_out, uint8_t* extra_starts,
@@ -653,14 +675,11 @@ __device__ __forceinline__ void update_walk_block(
   cp_async_wait_all();
   __syncthreads();
 
-  const bool word_ok = (reinterpret_cast<uintptr_t>(other) & 3u) == 0;
-  // A job table comes from the caller's device memory: an unaligned by-product pointer takes
-  // the scalar stores, a missing one is skipped.
-  BlockUpdate<kLaneMask, kEmit, kForm> work{
+  BlockUpdate<kLaneMask, kEmit, kForm, kAligned> work{
       g, Operation<kForm>(spec), block * g.steps, side_out + block_base + own_bytes(),
-      {other + block_base, left}, word_ok ? min(g.steps, left / kLanes) / kChunkRows * kChunkRows : 0,
+      {other + block_base, left}, min(g.steps, left / kLanes) / kChunkRows * kChunkRows,
       {dense_out == nullptr ? nullptr : dense_out + block_base, left},
-      (reinterpret_cast<uintptr_t>(dense_out) & 3u) == 0, spill + block_base, rows_used,
+      spill + block_base, rows_used,
       after_barrier(shared_address(own.encode_table)), (tid & 1) ? 0x4415u : 0x4440u, {}, {}, {}, {}};
   work.sides = sides;
   work.rows.open();
@@ -687,12 +706,20 @@ update_fused_batch_kernel(const lct_update_job* __restrict__ jobs, int n_jobs, S
     if (jobs[mid].first_block <= block) lo = mid; else hi = mid - 1;
   }
   const lct_update_job& job = jobs[lo];
-  update_walk_block<kLaneMask, kEmit, kForm>(
-      view_of_update(job.a), shape_of_update(job, common), static_cast<const uint16_t*>(job.other),
-      spec, shifted_encode + 256 * (int64_t)lo, job.side_out,
-      reinterpret_cast<uint32_t*>(job.encoded_out), extra_starts + job.first_block * kLanes,
-      summaries + 4 * job.first_block, job.spill, static_cast<uint16_t*>(job.dense_out),
-      block - job.first_block);
+  const auto run = [&](auto aligned) {
+    update_walk_block<kLaneMask, kEmit, kForm, decltype(aligned)::value>(
+        view_of_update(job.a), shape_of_update(job, common), static_cast<const uint16_t*>(job.other),
+        spec, shifted_encode + 256 * (int64_t)lo, job.side_out,
+        reinterpret_cast<uint32_t*>(job.encoded_out), extra_starts + job.first_block * kLanes,
+        summaries + 4 * job.first_block, job.spill, static_cast<uint16_t*>(job.dense_out),
+        block - job.first_block);
+  };
+  // A job table comes from the caller's device memory: a dense operand at an odd multiple of two
+  // bytes takes the unaligned form, and so does a by-product at one or a missing one (skipped).
+  uintptr_t bits = reinterpret_cast<uintptr_t>(job.other);
+  if (kEmit != LCT_EMIT_NONE) bits |= job.dense_out == nullptr ? 1u : reinterpret_cast<uintptr_t>(job.dense_out);
+  if ((bits & 3u) == 0) run(std::true_type());
+  else run(std::false_type());
 }
 
 using UpdateBatchKernel = void (*)(const lct_update_job*, int, Shape, OpSpec, const int32_t*,
