@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 import torch
 
-from gpu_helpers import bits_of, to_dev
+from gpu_helpers import assert_same_components, bits_of, to_dev
 from helpers import oracle_compress
 from losslessly_compressed_tensors_b200 import config
 from losslessly_compressed_tensors_b200.LCTensor import LCTTensor
@@ -62,6 +62,7 @@ def test_walk(oracle, n, codebook, kind):
     for got, want in zip(decompress_many([b, a]), (third, bits)):
         assert np.array_equal(bits_of(got), want)
     want_a = oracle_compress(oracle, bits, dist, oracle.new_arena(1 << 20))
+    assert_same_components(a, want_a)
     alpha = torch.tensor([0.95], dtype=torch.float32, device="cuda")
     wide = to_dev(right)
     for offset in (0, 1):  # the dense operand at 16 and at 2 bytes alignment
