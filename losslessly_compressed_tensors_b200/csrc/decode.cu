@@ -15,7 +15,7 @@
 // weights, a quarter of them the not-a-full-pair path).  Against the former form (16-row tiles
 // transposed through shared memory to eight columns per thread, 50 instructions), at 64 Mi
 // elements: 69.0 -> 59.3 us (weights with outliers), 58.8 -> 52.1 (normal), 60.6 -> 52.8 (half
-// zeros, overflow); 1 Mi: 11.3 -> 9.4.  Measured and left: two lanes per thread (90 us: half the
+// zeros, overflow); 1 Mi: 11.3 -> 9.4.  Measured and left: two lanes per thread (96 us: half the
 // warps, each with twice the serial chain), side bytes requested into registers (90 us: the loads'
 // registers spill, which waits for every load at once), 3 instead of 4 CTAs per SM (61.0).
 //

@@ -53,8 +53,8 @@ __device__ __forceinline__ uint32_t spread_exponents(uint32_t low, uint32_t high
 // One codec block.  extra_starts and summaries are the tensor's own arrays
 // (summaries holds g.n_blocks entries per row).
 // kLaneMask: the lane mapping as a compile-time constant (254, the default mapping), or -1 to
-// take it from the shape at run time.
-template <bool kPrecomputed, int kLaneMask>
+// take it from the shape at run time.  kAligned: the source's words of two values are aligned.
+template <bool kPrecomputed, int kLaneMask, bool kAligned>
 struct BlockEncoder {
   const char* rows;  // the block's first source row
   uint8_t* side_rows;
@@ -95,6 +95,11 @@ struct BlockEncoder {
       lanes[1].append(p.b0, p.b1);
     }
   }
+  // Bring rows of the source to L2, from the 16-byte granule on that holds the first one's start.
+  __device__ __forceinline__ void prefetch(int first_row, int count) const {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(rows) + (uint32_t)(first_row * kRowBytes);
+    prefetch_l2(reinterpret_cast<const void*>(at & ~(uintptr_t)15), count * kRowBytes);
+  }
   // The words of the chunk at step0, all requested together: loads requested one by one between
   // other work would make every use wait for the latest of them.
   __device__ __forceinline__ void request(uint32_t (&words)[kChunkRows], int step0) const {
@@ -111,7 +116,38 @@ struct BlockEncoder {
       }
     }
   }
-  // A word by guarded loads: a source of any alignment, a chunk that reaches past the end.
+  // Rows of a source at an odd multiple of two bytes, up to `full_rows`: a word is two loads of two
+  // bytes, requested a chunk ahead and joined when the chunk's turn comes.
+  __device__ __forceinline__ void run_unaligned(int full_rows, uint32_t budget_bits) {
+    uint32_t first[kChunkRows], second[kChunkRows];
+    auto request_values = [&](int step0) {
+      if (step0 >= full_rows) return;
+      const uint32_t offset = chunk_offset<kLaneMask>(block * g.steps, step0, g.lane_mask);
+#pragma unroll
+      for (int row = 0; row < kChunkRows; ++row) {
+        const char* p = rows + chunk_word<kLaneMask>(offset, row >> 1, g.lane_mask) + row * kRowBytes;
+        first[row] = load_ahead_u16(p);
+        second[row] = load_ahead_u16(p + 2);
+      }
+    };
+    request_values(0);
+#pragma unroll 1
+    for (int step0 = 0; step0 < full_rows; step0 += kChunkRows) {
+      Pair pairs[kChunkPairs];
+#pragma unroll
+      for (int k = 0; k < kChunkPairs; ++k)
+        pairs[k] = look_up(first[2 * k] | (second[2 * k] << 16), first[2 * k + 1] | (second[2 * k + 1] << 16));
+      request_values(step0 + kChunkRows);
+#pragma unroll
+      for (int k = 0; k < kChunkPairs; ++k) {
+        store_sides(pairs[k], k);
+        append<true>(pairs[k], step0 + 2 * k, budget_bits);
+      }
+      side_rows += kChunkRows * kLanes;
+    }
+  }
+
+  // A word by guarded loads: a chunk that reaches past the end, exponent bytes of any alignment.
   __device__ __forceinline__ uint32_t guarded_word(int step0, int k, bool second) const {
     const int64_t left = g.logical_numel - block * (int64_t)g.block_symbols;
     const uint32_t offset = chunk_offset<kLaneMask>(block * g.steps, step0, g.lane_mask);
@@ -159,7 +195,7 @@ struct BlockEncoder {
 #pragma unroll 1
     do {
       if (prefetches && step0 + kPrefetchRows + kPrefetchPortion <= wide_rows)
-        prefetch_l2(rows + (step0 + kPrefetchRows) * kRowBytes, kPrefetchPortion * kRowBytes);
+        prefetch(step0 + kPrefetchRows, kPrefetchPortion);
       if (near())
         step_chunk<true>(step0, now, even, odd, budget_bits);
       else
@@ -199,17 +235,18 @@ struct BlockEncoder {
   }
 
   // All rows up to `rows_used`: whole chunks as above, the rest by guarded loads.
-  __device__ __forceinline__ void run(int rows_used, bool prefetches) {
+  __device__ __forceinline__ void run(int rows_used, int full_rows, bool prefetches) {
     const uint32_t budget_bits = (uint32_t)g.fixed_words * 32u;
-    if (wide_rows > 0) {
+    if (kAligned && wide_rows > 0) {
       const int closed_from = run_open(prefetches, budget_bits);
       if (!kPrecomputed) run_closed(closed_from);
     }
+    if (!kAligned && !kPrecomputed) run_unaligned(full_rows, budget_bits);
     const int lane = 2 * threadIdx.x;
     const int valid_a = valid_steps_of(block, lane, g.steps, g.block_symbols, g.logical_numel, g.lane_mask);
     const int valid_b = valid_steps_of(block, lane + 1, g.steps, g.block_symbols, g.logical_numel, g.lane_mask);
 #pragma unroll 1
-    for (int step0 = wide_rows; step0 < rows_used; step0 += kChunkRows) {
+    for (int step0 = kPrecomputed ? wide_rows : full_rows; step0 < rows_used; step0 += kChunkRows) {
       Pair pairs[kChunkPairs];
 #pragma unroll
       for (int k = 0; k < kChunkPairs; ++k) {
@@ -231,9 +268,8 @@ struct BlockEncoder {
   }
 };
 
-template <bool kPrecomputed, int kLaneMask>
-__device__ __forceinline__ void encode_block(const void* __restrict__ src, bool src_word_ok,
-                                             uint8_t* __restrict__ side,
+template <bool kPrecomputed, int kLaneMask, bool kAligned>
+__device__ __forceinline__ void encode_block(const void* __restrict__ src, uint8_t* __restrict__ side,
                                              uint32_t* __restrict__ encoded,
                                              const int32_t* shifted_encode,
                                              uint8_t* __restrict__ extra_starts,
@@ -251,17 +287,16 @@ __device__ __forceinline__ void encode_block(const void* __restrict__ src, bool 
   // ragged or tiny tensor) carry no bits; their side bytes are cleared in one sweep.
   const int64_t left = g.logical_numel - block_base;
   const int in_block = (int)max((int64_t)0, min((int64_t)g.block_symbols, left));
-  const int full_rows = in_block / kLanes;
+  const int full_rows = in_block / (kChunkRows * kLanes) * kChunkRows;
   const int rows_used = (in_block + kChunkRows * kLanes - 1) / (kChunkRows * kLanes) * kChunkRows;
-  BlockEncoder<kPrecomputed, kLaneMask> encoder{
+  BlockEncoder<kPrecomputed, kLaneMask, kAligned> encoder{
       static_cast<const char*>(src) + block_base * (kPrecomputed ? 1 : 2),
       side + block_base + 2 * tid, g, block, 0u,
-      src_word_ok ? full_rows / kChunkRows * kChunkRows : 0, {}};
-  // A full block of an aligned source is fetched ahead; the first portions now, with everything
-  // up to the table still to come.
-  const bool prefetches = !kPrecomputed && tid == 0 && (reinterpret_cast<uintptr_t>(src) & 15u) == 0;
-  if (prefetches && encoder.wide_rows >= kPrefetchRows)
-    prefetch_l2(encoder.rows, kPrefetchRows * kRowBytes);
+      kAligned ? full_rows : 0, {}};
+  // A full block is fetched ahead; the first portions now, with everything up to the table still
+  // to come.
+  const bool prefetches = !kPrecomputed && tid == 0;
+  if (prefetches && encoder.wide_rows >= kPrefetchRows) encoder.prefetch(0, kPrefetchRows);
   clear_image<kPairThreads>(image, g.fixed_words);
   if (block == 0 && tid < 4) encoded[g.streams * g.fixed_words + tid] = 0u;  // trailing pad words
   if (!kPrecomputed && rows_used < g.steps) {
@@ -279,7 +314,7 @@ __device__ __forceinline__ void encode_block(const void* __restrict__ src, bool 
   encoder.lanes[0].open(shared_address(image + 2 * tid));
   encoder.lanes[1].open(shared_address(image + 2 * tid + 1));
   encoder.table = after_barrier(shared_address(sh.table));
-  encoder.run(rows_used, prefetches);
+  encoder.run(rows_used, full_rows, prefetches);
   finish_block<kPairThreads>(encoder.lanes, image, sh.scan, encoded, extra_starts, summaries, block,
                g.n_blocks, g.streams, g.steps, g.fixed_words);
 }
@@ -287,13 +322,12 @@ __device__ __forceinline__ void encode_block(const void* __restrict__ src, bool 
 // A closed lane must stay on the checked path: it closed within one pair (32 bits) of its budget.
 static_assert(kChunkBits >= 32, "a closed lane is near its budget");
 
-template <bool kPrecomputed, int kLaneMask>
+template <bool kPrecomputed, int kLaneMask, bool kAligned>
 __global__ void __launch_bounds__(kPairThreads, kEncodeMinCtas)
-encode_kernel(const void* __restrict__ src, bool src_word_ok, uint8_t* __restrict__ side,
-              uint32_t* __restrict__ encoded, const int32_t* shifted_encode,
+encode_kernel(const void* __restrict__ src, uint8_t* __restrict__ side, uint32_t* __restrict__ encoded, const int32_t* shifted_encode,
               uint8_t* __restrict__ extra_starts, int32_t* __restrict__ summaries, EncodeShape g) {
-  encode_block<kPrecomputed, kLaneMask>(src, src_word_ok, side, encoded, shifted_encode,
-                                        extra_starts, summaries, g, blockIdx.x);
+  encode_block<kPrecomputed, kLaneMask, kAligned>(src, side, encoded, shifted_encode, extra_starts,
+                                                  summaries, g, blockIdx.x);
 }
 
 // Shape of one job of a batch (all jobs share the geometry in `common`).
@@ -326,12 +360,14 @@ encode_batch_kernel(const lct_encode_job* __restrict__ jobs, int n_jobs,
   const int j = find_encode_job(jobs, n_jobs, block);
   const lct_encode_job& job = jobs[j];
   const EncodeShape g = shape_of_job(job, common);
-  const bool word_ok = (reinterpret_cast<uintptr_t>(job.src) & 3u) == 0;
-  encode_block<false, kLaneMask>(job.src, word_ok, job.side,
-                                 reinterpret_cast<uint32_t*>(job.encoded),
-                                 shifted_encode + 256 * (int64_t)j,
-                                 extra_starts + job.first_block * kLanes,
-                                 summaries + 4 * job.first_block, g, block - job.first_block);
+  const auto run = [&](auto aligned) {
+    encode_block<false, kLaneMask, decltype(aligned)::value>(
+        job.src, job.side, reinterpret_cast<uint32_t*>(job.encoded), shifted_encode + 256 * (int64_t)j,
+        extra_starts + job.first_block * kLanes, summaries + 4 * job.first_block, g,
+        block - job.first_block);
+  };
+  if ((reinterpret_cast<uintptr_t>(job.src) & 3u) == 0) run(std::true_type());
+  else run(std::false_type());
 }
 
 // Compact overflow metadata and raw exponent tails of one block.  Lanes are
@@ -472,20 +508,24 @@ static int launch_encode(const void* src, uint8_t* side, int32_t* encoded,
   if ((reinterpret_cast<uintptr_t>(encoded) & 15u) ||
       (!precomputed && (reinterpret_cast<uintptr_t>(side) & 15u)))
     return LCT_E_ALIGNMENT;
-  const bool word_ok = (s & (precomputed ? 1u : 3u)) == 0;
+  const bool aligned = (s & (precomputed ? 1u : 3u)) == 0;
   const size_t shared = sizeof(lct::EncodeSharedHead) + (size_t)fixed_words * lct::kLanes * 4;
   uint32_t* words = reinterpret_cast<uint32_t*>(encoded);
   const bool swizzled = g.lane_mask == 254;
-  auto kernel = precomputed ? (swizzled ? lct::encode_kernel<true, 254> : lct::encode_kernel<true, -1>)
-                            : (swizzled ? lct::encode_kernel<false, 254> : lct::encode_kernel<false, -1>);
+  // (Unaligned sources are rare: one kernel for both lane mappings serves them.)
+  auto kernel = precomputed ? (!aligned    ? lct::encode_kernel<true, -1, false>
+                               : swizzled  ? lct::encode_kernel<true, 254, true>
+                                           : lct::encode_kernel<true, -1, true>)
+                            : (!aligned    ? lct::encode_kernel<false, -1, false>
+                               : swizzled  ? lct::encode_kernel<false, 254, true>
+                                           : lct::encode_kernel<false, -1, true>);
   rc = (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
   if (rc) return rc;
   if (overlapped)
     return lct::launch_overlapped(kernel, (unsigned)g.n_blocks, lct::kPairThreads, shared, st, src,
-                                  word_ok, side, words, shifted_encode, extra_starts, summaries, g);
-  kernel<<<(unsigned)g.n_blocks, lct::kPairThreads, shared, st>>>(src, word_ok, side, words,
-                                                              shifted_encode, extra_starts,
-                                                              summaries, g);
+                                  side, words, shifted_encode, extra_starts, summaries, g);
+  kernel<<<(unsigned)g.n_blocks, lct::kPairThreads, shared, st>>>(src, side, words, shifted_encode,
+                                                              extra_starts, summaries, g);
   return (int)cudaGetLastError();
 }
 
